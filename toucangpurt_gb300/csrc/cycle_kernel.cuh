@@ -51,6 +51,31 @@ __device__ __forceinline__ unsigned long long dmix64(unsigned long long z) {
   return z ^ (z >> 31);
 }
 
+// Digest terms of one index of a pool: mix64(i << 8 | v) for several values v.
+// z = (i << 8) + C + v with the low byte of (i << 8) + C equal to 0x15, so a
+// value below 0xEB changes that byte only: z >> 30 and the upper 56 bits of
+// z ^ (z >> 30) depend on i alone, and the first multiplication splits into
+// (upper bits) * M1, done once per index, plus (low byte) * M1.
+constexpr unsigned long long kMixC = 0x9E3779B97F4A7C15ull, kMixM1 = 0xBF58476D1CE4E5B9ull,
+                             kMixM2 = 0x94D049BB133111EBull;
+struct MixIndex {
+  unsigned long long p;  // (upper 56 bits of z ^ (z >> 30)) * M1
+  uint32_t k;            // low byte of z >> 30
+  __device__ __forceinline__ explicit MixIndex(unsigned long long i) {
+    const unsigned long long z = (i << 8) + kMixC, s = z >> 30;
+    p = ((z ^ s) & ~0xFFull) * kMixM1;
+    k = uint32_t(s) & 0xFFu;
+  }
+  __device__ __forceinline__ unsigned long long operator()(uint32_t v) const { return term(p, k, v); }
+  // the term of value v (< 0xEB) from an index's p and k
+  static __device__ __forceinline__ unsigned long long term(unsigned long long p, uint32_t k, uint32_t v) {
+    const uint32_t b = (v + uint32_t(kMixC & 0xFFu)) ^ k;
+    unsigned long long y = p + (unsigned long long)b * kMixM1;
+    y = (y ^ (y >> 27)) * kMixM2;
+    return y ^ (y >> 31);
+  }
+};
+
 __device__ __forceinline__ void raiseErr(const KParams &p, uint32_t code, uint32_t a, uint32_t b, uint32_t c) {
   if (atomicCAS(p.err, 0u, code) == 0u) {
     p.errInfo[0] = code;

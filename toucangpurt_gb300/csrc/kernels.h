@@ -30,6 +30,8 @@ cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint
 cudaError_t launchInitState(int spw, const KParams &p, cudaStream_t st);
 cudaError_t launchRegDigest(int spw, const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t nStreams,
                             unsigned long long *out, cudaStream_t st);
+cudaError_t launchRegDigestOne(const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t g, uint32_t k,
+                               unsigned long long *out, cudaStream_t st);
 cudaError_t launchMemDigest(const uint8_t *mems, unsigned long long stride, uint32_t size, uint32_t nStreams,
                             unsigned long long *out, cudaStream_t st);
 cudaError_t launchGatherRegs(const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t g, uint32_t k, uint8_t *out,

@@ -1461,10 +1461,14 @@ int tgs_state_digest(tgs_sim *h, uint32_t s, uint64_t *rd, uint64_t *md) {
   return guard([&] {
     requireLoaded(h);
     if (s >= h->nStreams) throw Error(TGS_ERR_ARG, "stream index out of range");
-    TGS_CUDA(cudaMemsetAsync(h->outA.p, 0, h->nStreams * 8, h->stream));
-    TGS_CUDA(cudaMemsetAsync(h->outB.p, 0, h->nStreams * 8, h->stream));
-    TGS_CUDA(launchRegDigest(int(h->spw), h->regs.p, h->design.regPoolSize, h->gpad, h->nStreams, h->outA.p, h->stream));
-    TGS_CUDA(launchMemDigest(h->mems.p, h->memStride, h->design.memPoolSize, h->nStreams, h->outB.p, h->stream));
+    // the stream's own word of every register and its own memories
+    uint32_t g, k;
+    streamPos(h, s, g, k);
+    TGS_CUDA(cudaMemsetAsync(h->outA.p + s, 0, 8, h->stream));
+    TGS_CUDA(cudaMemsetAsync(h->outB.p + s, 0, 8, h->stream));
+    TGS_CUDA(launchRegDigestOne(h->regs.p, h->design.regPoolSize, h->gpad, g, k, h->outA.p + s, h->stream));
+    TGS_CUDA(launchMemDigest(h->mems.p + size_t(s) * h->memStride, h->memStride, h->design.memPoolSize, 1,
+                             h->outB.p + s, h->stream));
     unsigned long long a = 0, b = 0;
     TGS_CUDA(cudaMemcpyAsync(&a, h->outA.p + s, 8, cudaMemcpyDeviceToHost, h->stream));
     TGS_CUDA(cudaMemcpyAsync(&b, h->outB.p + s, 8, cudaMemcpyDeviceToHost, h->stream));
