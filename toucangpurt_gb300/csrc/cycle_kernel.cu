@@ -56,6 +56,22 @@ __global__ void initStateKernel(const KParams p) {
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < ne; i += size_t(gridDim.x) * blockDim.x) p.exg[i] = 0;
 }
 
+// Every stream's memories from the initial image: a thread reads 16 bytes
+// once and writes them to each stream of its block row (image and strides are
+// whole 16-byte pieces), so a reset writes each memory once and reads the
+// image once per kInitStreams streams instead of copying it per stream.
+// 16M-LUT design, 64 x 512 MiB: 10.4 ms -> 5.27 ms (6.5 TB/s written).
+constexpr uint32_t kInitStreams = 64;
+
+__global__ void __launch_bounds__(256) initMemsKernel(const uint8_t *__restrict__ init, uint8_t *__restrict__ mems,
+                                                     unsigned long long stride, uint32_t vecs, uint32_t nStreams) {
+  const uint32_t s0 = blockIdx.y * kInitStreams, s1 = min(nStreams, s0 + kInitStreams);
+  for (uint32_t v = blockIdx.x * 256u + threadIdx.x; v < vecs; v += gridDim.x * 256u) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4 *>(init) + v);
+    for (uint32_t s = s0; s < s1; ++s) __stcs(reinterpret_cast<uint4 *>(mems + s * stride) + v, w);
+  }
+}
+
 // Digest of one pool per stream: sum over i of mix64(i << 8 | v_i).
 // A block takes up to kDigestStreams streams, a thread the same 16 bytes of
 // each of them.  Streams' memories start equal and are written sparsely, so a
@@ -322,6 +338,15 @@ cudaError_t launchInitState(int spw, const KParams &p, cudaStream_t st) {
     initStateKernel<8><<<blocks, 256, 0, st>>>(p);
   else
     initStateKernel<1><<<blocks, 256, 0, st>>>(p);
+  return cudaGetLastError();
+}
+
+cudaError_t launchInitMems(const KParams &p, cudaStream_t st) {
+  const uint32_t vecs = uint32_t((size_t(p.memPoolSize) + 15) / 16);
+  if (!vecs) return cudaSuccess;
+  const uint32_t gy = (p.nStreams + kInitStreams - 1) / kInitStreams;
+  dim3 grid(std::min<uint32_t>((vecs + 255) / 256, std::max<uint32_t>(1, 4864u / gy)), gy);
+  initMemsKernel<<<grid, 256, 0, st>>>(p.initMems, p.mems, p.memStride, vecs, p.nStreams);
   return cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@ cudaError_t enqueueGraphChunk(const LaunchCfg &c, const KParams &p, uint32_t k, 
 cudaError_t launchStimulus(int spw, const KParams &p, uint32_t cycle, cudaStream_t st);
 cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n);
 cudaError_t launchInitState(int spw, const KParams &p, cudaStream_t st);
+cudaError_t launchInitMems(const KParams &p, cudaStream_t st);
 cudaError_t launchRegDigest(int spw, const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t nStreams,
                             unsigned long long *out, cudaStream_t st);
 cudaError_t launchRegDigestOne(const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t g, uint32_t k,

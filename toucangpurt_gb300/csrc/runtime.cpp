@@ -490,9 +490,7 @@ void configure(tgs_sim *h) {
 
 void resetState(tgs_sim *h) {
   TGS_CUDA(launchInitState(int(h->spw), h->kp, h->stream));
-  for (uint32_t s = 0; s < h->nStreams; ++s)
-    TGS_CUDA(cudaMemcpyAsync(h->mems.p + size_t(s) * h->memStride, h->initMems.p, h->design.memPoolSize,
-                             cudaMemcpyDeviceToDevice, h->stream));
+  TGS_CUDA(launchInitMems(h->kp, h->stream));
   TGS_CUDA(cudaMemsetAsync(h->stop.p, 0, h->nStreams * sizeof(uint32_t), h->stream));
   TGS_CUDA(cudaMemsetAsync(h->stopCycle.p, 0xFF, h->nStreams * sizeof(uint32_t), h->stream));
   TGS_CUDA(cudaMemsetAsync(h->realCycles.p, 0, sizeof(uint32_t), h->stream));
