@@ -10,7 +10,6 @@ namespace tgs {
 
 constexpr int kMlpParams = 64 * 16 + 64 + 64 * 64 + 64 + 64 + 1;  // 5,313
 
-size_t mlpGradSmem();
 // out[i] = network(X[i]) for n samples of 16 features (device pointers)
 cudaError_t mlpForward(const float *params, const float *X, uint32_t n, float *out, cudaStream_t st);
 // grad += d/dparams of scale * sum_i (network(X[idx[i]]) - y[idx[i]])^2 ; loss += the sum of squares
