@@ -325,7 +325,7 @@ def levels_option(a) -> int:
 
 
 def exec_levels(st) -> str:
-    return "resident" if st.get("resident_words") else "staged" if st.get("stage_words") else "global"
+    return "warp programs" if st.get("program_words") else "resident" if st.get("resident_words") else "staged" if st.get("stage_words") else "global"
 
 
 def make_simulator(a, dp, sp, streams, gpu):

@@ -67,10 +67,12 @@ typedef struct tgs_options {
   uint32_t mode;             /* TGS_MODE_PERSISTENT or TGS_MODE_GRAPH */
   uint32_t barrier_timeout_ms; /* budget of every device-side wait (default 2000) */
   uint32_t validate;         /* 1 = run the static design checks at init (default 1) */
-  uint32_t resident_netlist; /* 0 (default): a block's exec levels stay in shared memory for the whole launch when
-                                every block of the launch still fits on the GPU at once, else each level is staged
-                                into shared memory while the previous one runs; 1: resident (TGS_ERR_RESOURCES when
-                                it does not fit); 2: levels read from global memory; 3: staged */
+  uint32_t resident_netlist; /* 0 (default): each warp reads its part of the exec levels as one list of records,
+                                ahead of their use, into registers (value_pool = 1: as 1 when every block of the
+                                launch still fits on the GPU at once, else as 3); 1: a block's exec levels stay in
+                                shared memory for the whole launch (TGS_ERR_RESOURCES when they do not fit);
+                                2: levels read from global memory; 3: each level staged into shared memory while the
+                                previous one runs */
   uint32_t value_pool;       /* 0: renumber value-pool slots by live range (default); 1: the design file's numbering.
                                 Takes effect at the next tgs_init / tgs_init_from_memory */
   uint32_t capture_signals;  /* 1: record every signal of the symbol file each cycle (tgs_read_signal, VCD);
@@ -118,7 +120,7 @@ typedef struct tgs_tune_opts {
 
 typedef struct tgs_tune_trial {
   uint32_t groups_per_item, warps_per_block, blocks_per_sm, mode;
-  uint32_t staged;      /* exec levels: 1 staged per level, 2 resident for the launch, 0 read from global memory */
+  uint32_t staged;      /* exec levels: 1 staged per level, 2 resident for the launch, 0 read from global memory, 3 warp programs */
   uint32_t blocks;      /* grid size of the trial */
   float ms_per_cycle;   /* negative: the configuration does not fit */
   uint32_t mpart_lanes, levels_per_barrier;
@@ -334,7 +336,9 @@ typedef struct tgs_design_stats {
   uint32_t stage_words;      /* words of one exec-level stage buffer (0: levels resident or read from global memory) */
   uint32_t resident_words;   /* words of a block's resident exec levels (0: staged or read from global memory) */
   uint32_t fused_levels;     /* exec levels merged into the block before them (levels_per_barrier > 1) */
-  uint32_t reserved[4];
+  uint32_t program_words;    /* words of the warp programs (0: exec levels resident, staged or global) */
+  uint32_t region_items;     /* (partition, group block) items of the larger region */
+  uint32_t reserved[2];
 } tgs_design_stats;
 int tgs_get_design_stats(const tgs_sim *h, tgs_design_stats *out);
 

@@ -270,26 +270,30 @@ __global__ void peekRegsKernel(const uint32_t *__restrict__ regs, uint32_t gpad,
 
 }  // namespace
 
-void *cycleKernelFor(int spw, int G, bool resident) {
-  return resident ? cycleKernelResident(spw, G) : cycleKernelStaged(spw, G);
+void *cycleKernelFor(int spw, int G, int lv) {
+  return lv == kLevelsProgram    ? cycleKernelProgram(spw, G)
+         : lv == kLevelsResident ? cycleKernelResident(spw, G)
+                                 : cycleKernelStaged(spw, G);
 }
 
 cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n) {
-  void *fn = cycleKernelFor(c.spw, c.G, c.res);
+  void *fn = cycleKernelFor(c.spw, c.G, c.lv);
   KParams pp = p;
   void *args[] = {&pp, &c0, &n};
   return cudaLaunchCooperativeKernel(fn, dim3(c.blocks), dim3(c.threads), args, c.smem, c.stream);
 }
 
-void *regionKernelFor(int spw, int G, bool resident) {
-  return resident ? regionKernelResident(spw, G) : regionKernelStaged(spw, G);
+void *regionKernelFor(int spw, int G, int lv) {
+  return lv == kLevelsProgram    ? regionKernelProgram(spw, G)
+         : lv == kLevelsResident ? regionKernelResident(spw, G)
+                                 : regionKernelStaged(spw, G);
 }
 
 // Enqueues one chunk of k cycles in graph form on the stream (captured by
 // the caller): per cycle region 0, region 1 and (admission / cycle count)
 // the admit kernel; then the cycle counter advance.
 cudaError_t enqueueGraphChunk(const LaunchCfg &c, const KParams &p, uint32_t k, bool admit) {
-  void *fn = regionKernelFor(c.spw, c.G, c.res);
+  void *fn = regionKernelFor(c.spw, c.G, c.lv);
   KParams pp = p;
   for (uint32_t i = 0; i < k; ++i) {
     for (uint32_t r = 0; r < 2; ++r) {

@@ -376,12 +376,7 @@ __device__ __forceinline__ void evalLutPass(const Words<SH> mp, uint32_t hdr, ui
   }
   // middle levels: operand < 32 immediate, 32..63 = lane (op - 32) of the previous level
   const Words<SH> mid = top.at(2u * W);
-  // each level's op word is read one level ahead, so its latency overlaps
-  // the previous level's shuffles and lookups
-  uint32_t wNext = nMid && lane < W ? mid[lane] : 0u;
-  for (uint32_t m = 0; m < nMid; ++m) {
-    const uint32_t w = wNext;
-    wNext = m + 1 < nMid && lane < W ? mid[(m + 1) * W + lane] : 0u;
+  auto midStep = [&](uint32_t w) {
     const uint32_t c6 = w & 63u, b6 = (w >> 6) & 63u, a6 = (w >> 12) & 63u, lut = w >> 18;
     uint32_t nv[H];
 #pragma unroll
@@ -396,6 +391,30 @@ __device__ __forceinline__ void evalLutPass(const Words<SH> mp, uint32_t hdr, ui
     }
 #pragma unroll
     for (int g = 0; g < H; ++g) v[g] = nv[g];
+  };
+  if constexpr (!SH && H == 1) {
+    // one group, record in global memory: the op words of four levels are in
+    // flight (a level of one group takes about 200 cycles, an L2 read 700)
+    uint32_t q[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) q[j] = j < nMid && lane < W ? mid[j * W + lane] : 0u;
+    for (uint32_t m = 0; m < nMid; m += 4)
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) {
+        if (m + j >= nMid) break;
+        const uint32_t w = q[j];
+        q[j] = m + j + 4 < nMid && lane < W ? mid[(m + j + 4) * W + lane] : 0u;
+        midStep(w);
+      }
+  } else {
+    // each level's op word is read one level ahead, so its latency overlaps
+    // the previous level's shuffles and lookups
+    uint32_t wNext = nMid && lane < W ? mid[lane] : 0u;
+    for (uint32_t m = 0; m < nMid; ++m) {
+      const uint32_t w = wNext;
+      wNext = m + 1 < nMid && lane < W ? mid[(m + 1) * W + lane] : 0u;
+      midStep(w);
+    }
   }
   // write-back (SimEval.cu:422-447): shuffleId < 32 immediate, else lane
   // (shuffleId mod 32); a compact record's lane l writes its own value
@@ -638,6 +657,17 @@ __device__ __forceinline__ void stageCopy(const Stage &st, uint32_t b, const uin
 }
 __device__ __forceinline__ void stageCopyWait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// A micro-partition's record for the stream groups [g0, g0 + gn) of the item.
+template <int SPW, int G, bool SH>
+__device__ __forceinline__ void runRecord(const KParams &p, const PartDesc &d, const Words<SH> mp, uint32_t hdr,
+                                          uint32_t g0, uint32_t gn, uint32_t vp, uint32_t tab, uint32_t lane,
+                                          uint32_t gb) {
+  if ((hdr & 3u) == kMPLut) evalLut<SPW, G, SH>(mp, hdr, vp, tab, lane, p.constSlots != 0);  // always every group
+  else if ((hdr & 3u) == kMPVecRead) evalVecRead<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn);
+  else if ((hdr & 3u) == kMPVecOp) evalVecOp<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn);
+  else evalMemRead<SPW, G, SH>(p, mp, hdr, vp, lane, gb, g0, gn);
+}
+
 // The units a warp runs in one exec level (block = the level's words).
 // Unit u of a level block (unit word: record offset | first group << 24 |
 // (groups - 1) << 27).
@@ -647,14 +677,7 @@ __device__ __forceinline__ void runUnit(const KParams &p, const PartDesc &d, con
   const uint32_t uw = units[u];
   const Words<SH> mp = blk.at(uw & kUnitOffsetMask);
   const uint32_t hdr = mp[0];
-  if ((hdr & 3u) == kMPLut) {
-    evalLut<SPW, G, SH>(mp, hdr, vp, tab, lane, p.constSlots != 0);  // always every group
-  } else {
-    const uint32_t g0 = (uw >> 24) & 7u, gn = ((uw >> 27) & 7u) + 1u;
-    if ((hdr & 3u) == kMPVecRead) evalVecRead<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn);
-    else if ((hdr & 3u) == kMPVecOp) evalVecOp<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn);
-    else evalMemRead<SPW, G, SH>(p, mp, hdr, vp, lane, gb, g0, gn);
-  }
+  runRecord<SPW, G, SH>(p, d, mp, hdr, (uw >> 24) & 7u, ((uw >> 27) & 7u) + 1u, vp, tab, lane, gb);
   __syncwarp();
 }
 
@@ -685,12 +708,7 @@ __device__ __forceinline__ void runLevel(const KParams &p, const PartDesc &d, co
     const uint32_t g0 = (uw >> 24) & 7u, gn = ((uw >> 27) & 7u) + 1u;
     const uint32_t hdr = mp[0];
     const long long tm = clock64();
-    switch (hdr & 3u) {
-      case kMPLut: evalLut<SPW, G, SH>(mp, hdr, vp, tab, lane, p.constSlots != 0); break;
-      case kMPVecRead: evalVecRead<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn); break;
-      case kMPVecOp: evalVecOp<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn); break;
-      default: evalMemRead<SPW, G, SH>(p, mp, hdr, vp, lane, gb, g0, gn); break;
-    }
+    runRecord<SPW, G, SH>(p, d, mp, hdr, g0, gn, vp, tab, lane, gb);
     __syncwarp();
     if (lane == 0) {
       const uint32_t id = mp[1];
@@ -894,6 +912,102 @@ __device__ __forceinline__ void runLevelsSingle(const KParams &p, const PartDesc
   }
 }
 
+// ---- warp programs -----------------------------------------------------------
+// A warp's part of all exec levels of a partition as one list of 256-byte
+// entries (devimage.h), read into registers kProgAhead entries early: no level
+// descriptors, unit lists, headers or staged copies are left between a level
+// barrier and the operand loads, and a warp that has less to do in a level
+// only waits at its barrier.  The staged levels spent 240 of 380 warp
+// instructions of a 32-lane, 4-group record on these (16M-LUT design x 64
+// streams; without any table lookup they still took 42 of 62 ms); a record now
+// takes 225, and a region 135 M instead of 229 M.  Bound now by the
+// shared-memory pipe (bank conflicts of random table reads and operands, 78-83 %
+// of its cycles).  Per 100 cycles: 61.0 -> 47.8 ms; 1M-LUT design x 64 streams
+// 7.8 -> 5.6 ms, one stream 300 cycles 7.9 -> 6.0 ms; 4K-LUT design, one stream,
+// 1,000 cycles (levels resident before) 9.4 -> 6.4 ms.
+struct ProgOps {
+  uint32_t aA, aB, aC, aR, lut;  // operand and result addresses of the item's first group, lut field
+};
+
+template <int G>
+__device__ __forceinline__ ProgOps decodeEntry(uint2 w, uint32_t vp) {
+  constexpr uint32_t kSlot = 4u * G;
+  ProgOps o;
+  o.aA = vp + (w.x >> 20) * kSlot;
+  o.aB = vp + ((w.x >> 8) & 0xFFFu) * kSlot;
+  o.aC = vp + (w.y >> 20) * kSlot;
+  o.aR = vp + ((w.y >> 8) & 0xFFFu) * kSlot;
+  o.lut = (w.x & 0xFFu) | (w.y & 0xF8u) << 5;
+  return o;
+}
+
+template <int SPW, int G, bool PROF>
+__device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, uint2 begin, uint2 r0, uint2 r1,
+                                           uint32_t vp, uint32_t tab, uint32_t lane, uint32_t gb) {
+  constexpr int H = G > 4 ? 4 : G;
+  const uint2 *next = p.prog + size_t(begin.x + kProgAhead) * 32u + lane;
+  ProgOps o = decodeEntry<G>(r0, vp);
+  uint2 w = r0;
+  for (uint32_t e = 0; e < begin.y; ++e) {
+    const uint2 w1 = r1;
+    r1 = __ldg(next);
+    next += 32;
+    const uint32_t kind = w.y & 3u;
+    long long tm = 0;
+    if constexpr (PROF) tm = clock64();
+    uint32_t gn = G;
+    if (kind == kProgTable) {
+#pragma unroll
+      for (int h = 0; h < G; h += H) {
+        uint32_t A[H], B[H], C[H], v[H];
+        loadG<H>(o.aA + 4u * h, A);
+        loadG<H>(o.aB + 4u * h, B);
+        loadG<H>(o.aC + 4u * h, C);
+#pragma unroll
+        for (int g = 0; g < H; ++g) {
+          const uint32_t T = lookup<SPW>(tab, o.lut, A[g], B[g], C[g]);
+          v[g] = o.lut ? T : C[g];
+        }
+        storeG<H>(o.aR + 4u * h, v);
+      }
+    } else if (kind != kProgUnit) {
+      if constexpr (SPW == 8) {
+#pragma unroll
+        for (int h = 0; h < G; h += H) {
+          uint32_t A[H], B[H], C[H], v[H];
+          loadG<H>(o.aB + 4u * h, B);
+          loadG<H>(o.aC + 4u * h, C);
+          if (kind == kProgMux) {
+            loadG<H>(o.aA + 4u * h, A);
+            fastTop<H>(tab, o.lut & 0x3FFu, o.lut >> 11, o.lut & 15u, A, B, C, v, true);
+          } else {
+            fastTop<H>(tab, 0u, 0u, o.lut, A, B, C, v, false);
+          }
+          storeG<H>(o.aR + 4u * h, v);
+        }
+      }
+    } else {
+      gn = (w.y >> 16) & 15u;
+      if (gn) {
+        const Words<false> mp{p.net + w.x, 0u};
+        runRecord<SPW, G, false>(p, d, mp, mp[0], (w.y >> 12) & 15u, gn, vp, tab, lane, gb);
+      }
+    }
+    __syncwarp();
+    if constexpr (PROF) {
+      if (lane == 0 && gn) {
+        const uint32_t id = __ldg(p.progId + begin.x + e);
+        atomicAdd(p.mpCycles + id, (unsigned long long)(clock64() - tm));
+        atomicAdd(p.mpCount + id, gn);  // groups evaluated
+      }
+    }
+    // the next entry's addresses are ready before the barrier
+    o = decodeEntry<G>(w1, vp);
+    if (w.y & kProgBarrier) __syncthreads();
+    w = w1;
+  }
+}
+
 // ---- one partition for G groups (evalEachPartition, SimEval.cu:765-864) ---
 // vp, tab: shared addresses of the block's value pool and truth table.
 __device__ __forceinline__ PartDesc loadPart(const PartDesc *pd) {
@@ -931,7 +1045,7 @@ __device__ bool residentWait(const KParams &p, uint32_t mb) {
 // (0: staged or read from global memory); resState: 0 levels not resident
 // (or their copies timed out), 1 copies issued and not yet waited for, 2
 // resident levels ready.
-template <int SPW, int G, bool RES>
+template <int SPW, int G, int LV>
 __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t tab, Stage &st, uint32_t cycle,
                          const uint32_t *retire, uint32_t res, uint32_t &resState) {
   const uint32_t pid = item & 0xFFFFFu, gb = item >> 20;
@@ -939,13 +1053,21 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   // stores (whose memory clobber would otherwise force global reloads)
   const PartDesc d = loadPart(p.parts + pid);
   const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, warp = tid >> 5, NW = nthr >> 5;
-  const uint2 *__restrict__ ld = p.levelDesc + d.schedOff;
-  const uint32_t cap = p.stageWords;
+  constexpr bool RES = LV == kLevelsResident, PROG = LV == kLevelsProgram;
+  // warp program: the first entries are on their way while the level-0 reads run
+  uint2 begin = make_uint2(0u, 0u), r0 = begin, r1 = begin;
+  if constexpr (PROG) {
+    begin = __ldg(p.progBegin + pid * NW + warp);
+    r0 = __ldg(p.prog + size_t(begin.x) * 32u + lane);
+    r1 = __ldg(p.prog + size_t(begin.x + 1u) * 32u + lane);
+  }
+  const uint2 *__restrict__ ld = PROG ? nullptr : p.levelDesc + d.schedOff;
+  const uint32_t cap = PROG ? 0u : p.stageWords;
   // level descriptors (block offset, words) are loaded two levels ahead so
   // their latency stays off the per-level path
   const uint2 zero2 = make_uint2(0u, 0u);
-  uint2 cur = d.nLevels > 0 ? __ldg(ld) : zero2;
-  uint2 nxt = d.nLevels > 1 ? __ldg(ld + 1) : zero2;
+  uint2 cur = !PROG && d.nLevels > 0 ? __ldg(ld) : zero2;
+  uint2 nxt = !PROG && d.nLevels > 1 ? __ldg(ld + 1) : zero2;
   const uint32_t x0 = cur.x;  // first level block of the partition (resident offset 0)
   // the first exec level streams in while the level-0 reads run
   // (the block's last warp issues the pieces: the other warps go straight
@@ -975,13 +1097,20 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   }
 
   // exec levels: warp w runs the units the schedule gave it
-  bool levelsDone = false;
+  bool levelsDone = PROG;
+  if constexpr (PROG) {
+    if (p.flags & kFlagProfileMP)
+      runProgram<SPW, G, true>(p, d, begin, r0, r1, vp, tab, lane, gb);
+    else
+      runProgram<SPW, G, false>(p, d, begin, r0, r1, vp, tab, lane, gb);
+  }
   if constexpr (G == 1 && RES) {
     if (res && !(p.flags & kFlagProfileMP)) {
       runLevelsSingle<SPW>(p, d, res, x0, ld, cur, nxt, vp, tab, lane, warp, NW, gb);
       levelsDone = true;
     }
   }
+  if constexpr (!PROG)
   for (uint32_t lv = 0; lv < d.nLevels && !levelsDone; ++lv) {
     const uint2 after = lv + 2 < d.nLevels ? __ldg(ld + lv + 2) : zero2;
     bool staged = false;
@@ -1592,7 +1721,7 @@ __device__ __forceinline__ bool setupBlock(const KParams &p, uint8_t *smem, unsi
 // One region of cycle t for this block: its items, then the region's side
 // work (digests and retiring-stream capture in region 0; memory reset of
 // retiring streams, next cycle's inputs and digest folding in region 1).
-template <int SPW, int G, bool RES>
+template <int SPW, int G, int LV>
 __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t r, bool event, const uint32_t *retBits,
                            uint32_t retCnt, uint32_t cEnd, uint32_t c0) {
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
@@ -1601,8 +1730,8 @@ __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t 
   for (uint32_t i = i0; i < i1; ++i) {
     const long long tk = clock64();
     const uint32_t item = __ldg(p.items + i);
-    const uint32_t res = RES && p.resWords ? b.res + 4u * __ldg(p.itemRes + i) : 0u;
-    evalItem<SPW, G, RES>(p, item, b.vp, b.tab, b.st, t, (event && r == 1) ? p.retireMask : nullptr, res, b.resState);
+    const uint32_t res = LV == kLevelsResident && p.resWords ? b.res + 4u * __ldg(p.itemRes + i) : 0u;
+    evalItem<SPW, G, LV>(p, item, b.vp, b.tab, b.st, t, (event && r == 1) ? p.retireMask : nullptr, res, b.resState);
     // per-partition clock64 profile (SimEval.cu:894-983): running mean of the
     // useful ticks over cycles [100, 200) of a launch, group block 0
     if ((p.flags & kFlagProfile) && threadIdx.x == 0 && (item >> 20) == 0 && t >= c0 + 100 && t < c0 + 200) {
@@ -1626,13 +1755,13 @@ __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t 
 // cycle's inputs, (a retirement) admission; the launch ends early once every
 // queued stream retired or, resident streams with stop exit, every stream
 // stopped.
-template <int SPW, int G, bool RES>
+template <int SPW, int G, int LV>
 __global__ void __launch_bounds__(1024) cycleKernel(const KParams p, uint32_t c0, uint32_t nCycles) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) unsigned long long stageMbar[2];
   __shared__ uint32_t retBits[kMaxSlotWords];
   BlockSmem b;
-  if (!setupBlock<G, RES>(p, smem, stageMbar, b, -1)) return;
+  if (!setupBlock<G, LV == kLevelsResident>(p, smem, stageMbar, b, -1)) return;
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
   const uint32_t cEnd = c0 + nCycles;
   uint32_t gen = 0;
@@ -1649,7 +1778,7 @@ __global__ void __launch_bounds__(1024) cycleKernel(const KParams p, uint32_t c0
 #pragma unroll 1
     for (uint32_t r = 0; r < 2; ++r) {
       const long long tStart = clock64();
-      regionWork<SPW, G, RES>(p, b, t, r, event, retBits, retCnt, cEnd, c0);
+      regionWork<SPW, G, LV>(p, b, t, r, event, retBits, retCnt, cEnd, c0);
       if (!gridSync(p, gen)) return;
       if ((p.flags & kFlagProfile) && threadIdx.x == 0 && t >= c0 + 100 && t < c0 + 200) {
         const long long total = clock64() - tStart;
@@ -1684,7 +1813,7 @@ __global__ void __launch_bounds__(1024) cycleKernel(const KParams p, uint32_t c0
 
 // Graph form: one launch per region, kernel boundaries instead of the grid
 // barrier; cycle = device counter + k so one captured chunk is replayed.
-template <int SPW, int G, bool RES>
+template <int SPW, int G, int LV>
 __global__ void __launch_bounds__(1024) regionKernel(const KParams p, uint32_t k, uint32_t r) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) unsigned long long stageMbar[2];
@@ -1696,7 +1825,7 @@ __global__ void __launch_bounds__(1024) regionKernel(const KParams p, uint32_t k
   // admission words, loaded before the block setup hides their latency
   const uint32_t adm = !slots ? 0u : r == 0 ? __ldcg(p.eventHint + (t & 1u)) : __ldcg(p.retCount);
   BlockSmem b;
-  if (!setupBlock<G, RES>(p, smem, stageMbar, b, int(r))) return;
+  if (!setupBlock<G, LV == kLevelsResident>(p, smem, stageMbar, b, int(r))) return;
   uint32_t retCnt = adm;
   if (slots && r == 0) {
     retCnt = 0;
@@ -1705,28 +1834,27 @@ __global__ void __launch_bounds__(1024) regionKernel(const KParams p, uint32_t k
     else if (blockIdx.x == 0 && threadIdx.x == 0)
       p.eventHint[(t + 1u) & 1u] = adm;  // carried to the next cycle's launch
   }
-  regionWork<SPW, G, RES>(p, b, t, r, retCnt > 0, retBits, retCnt, cEnd, __ldcg(p.graphState + 3));
+  regionWork<SPW, G, LV>(p, b, t, r, retCnt > 0, retBits, retCnt, cEnd, __ldcg(p.graphState + 3));
 }
 
 // Kernel pointers by (streams per word, groups per item) for one exec-level
-// source (RES: resident for the launch; else staged per level or global);
-// each instantiating translation unit takes one form and one RES.
-template <bool RES>
+// source; each instantiating translation unit takes one form and one source.
+template <int LV>
 void *cycleKernelPtrT(int spw, int G) {
-  if (spw == 1) return reinterpret_cast<void *>(&cycleKernel<1, 1, RES>);
-  if (G == 8) return reinterpret_cast<void *>(&cycleKernel<8, 8, RES>);
-  if (G == 4) return reinterpret_cast<void *>(&cycleKernel<8, 4, RES>);
-  if (G == 2) return reinterpret_cast<void *>(&cycleKernel<8, 2, RES>);
-  return reinterpret_cast<void *>(&cycleKernel<8, 1, RES>);
+  if (spw == 1) return reinterpret_cast<void *>(&cycleKernel<1, 1, LV>);
+  if (G == 8) return reinterpret_cast<void *>(&cycleKernel<8, 8, LV>);
+  if (G == 4) return reinterpret_cast<void *>(&cycleKernel<8, 4, LV>);
+  if (G == 2) return reinterpret_cast<void *>(&cycleKernel<8, 2, LV>);
+  return reinterpret_cast<void *>(&cycleKernel<8, 1, LV>);
 }
 
-template <bool RES>
+template <int LV>
 void *regionKernelPtrT(int spw, int G) {
-  if (spw == 1) return reinterpret_cast<void *>(&regionKernel<1, 1, RES>);
-  if (G == 8) return reinterpret_cast<void *>(&regionKernel<8, 8, RES>);
-  if (G == 4) return reinterpret_cast<void *>(&regionKernel<8, 4, RES>);
-  if (G == 2) return reinterpret_cast<void *>(&regionKernel<8, 2, RES>);
-  return reinterpret_cast<void *>(&regionKernel<8, 1, RES>);
+  if (spw == 1) return reinterpret_cast<void *>(&regionKernel<1, 1, LV>);
+  if (G == 8) return reinterpret_cast<void *>(&regionKernel<8, 8, LV>);
+  if (G == 4) return reinterpret_cast<void *>(&regionKernel<8, 4, LV>);
+  if (G == 2) return reinterpret_cast<void *>(&regionKernel<8, 2, LV>);
+  return reinterpret_cast<void *>(&regionKernel<8, 1, LV>);
 }
 
 }  // namespace

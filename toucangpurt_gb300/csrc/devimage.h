@@ -91,8 +91,32 @@ static_assert(sizeof(PartDesc) == 96, "PartDesc size");
 // are copied there once per launch and stay resident (a partition's level
 // blocks are contiguous in KParams::sched).
 
+// Warp programs (KParams::prog), the streamed form of the exec levels: for
+// every partition and warp one list of entries of 32 lane words pairs (256 B),
+// read in order from global memory into registers two entries ahead.  Bits
+// 0..1 of the second word: kind, bit 2: a block barrier follows the entry
+// (the same bits in every lane).
+//   kProgTable, kProgWide, kProgMux: a compact LUT record with slot operands;
+//     lane l: [op0 << 20 | op1 << 8 | lut & 255, op2 << 20 | result << 8 |
+//     (lut >> 8) << 3 | bits]; lanes without an op repeat lane 0's.
+//     lut: lutIndex (table records), else lane kind << 11 | (kind 0: g, else
+//     the window's lutIndex, which is below 1,024)
+//   kProgUnit: any other micro-partition: [word offset of its record in
+//     KParams::net, (groups << 16) | (first group << 12) | bits]; groups = 0:
+//     nothing but the barrier
+enum : uint32_t { kProgTable = 0, kProgWide = 1, kProgMux = 2, kProgUnit = 3 };
+constexpr uint32_t kProgBarrier = 4u, kProgAhead = 2u;
+
+// Where a block reads its exec levels: staged per level into shared memory
+// (or, level by level, from global memory), resident there for the launch, or
+// warp programs.
+enum : int { kLevelsStaged = 0, kLevelsResident = 1, kLevelsProgram = 2 };
+
 // Kernel parameters (passed by value).
 struct KParams {
+  const uint2 *prog;          // warp programs (kLevelsProgram)
+  const uint2 *progBegin;     // (first entry, entries) per partition and warp
+  const uint32_t *progId;     // micro-partition id per entry (profiling)
   const uint32_t *net;        // design words
   const uint32_t *sched;      // exec-level blocks
   const uint2 *levelDesc;     // (block offset, words) per partition level

@@ -627,6 +627,62 @@ struct Dsu {
   void join(uint32_t a, uint32_t b) { p[find(a)] = find(b); }
 };
 
+// One entry of a warp program (devimage.h).
+struct ProgEntry {
+  uint32_t w[64];
+  uint32_t id;
+};
+
+void encodeEntry(const uint32_t *net, const MPartRef &m, uint32_t g0, uint32_t gn, uint32_t spw, ProgEntry &e) {
+  const uint32_t *r = net + m.off, hdr = r[0], W = (hdr >> 2) & 63u;
+  e.id = m.id;
+  if ((hdr & 3u) != kMPLut || !(hdr & kMPCompact)) {
+    for (uint32_t l = 0; l < 32; ++l) {
+      e.w[2 * l] = m.off;
+      e.w[2 * l + 1] = gn << 16 | g0 << 12 | kProgUnit;
+    }
+    return;
+  }
+  const bool fast = (hdr & kMPFastTop) != 0, wide = fast && spw > 1;
+  const uint32_t kind = !wide ? kProgTable : (hdr & kMPFastSel) ? kProgMux : kProgWide;
+  for (uint32_t l = 0; l < 32; ++l) {
+    const uint32_t *p = r + kMPHeaderWords + 2 * (l < W ? l : 0u);
+    uint32_t a = p[0] & 0xFFFu, lut = p[1] >> 16;
+    const uint32_t b = (p[0] >> 12) & 0xFFFu, c = (p[0] >> 24) | (p[1] & 15u) << 8, res = (p[1] >> 4) & 0xFFFu;
+    if (fast) {
+      const uint32_t laneKind = (lut >> kFastKindShift) & 3u;
+      lut &= (1u << kFastKindShift) - 1u;
+      if (wide) {
+        if (laneKind == 0) {
+          lut = (a >> 4) & 15u;
+          a = 0;  // an immediate: never read
+        } else {
+          lut |= laneKind << 11;
+        }
+      } else if (laneKind == 0) {
+        a &= 15u;
+      }
+    }
+    e.w[2 * l] = a << 20 | b << 8 | (lut & 0xFFu);
+    e.w[2 * l + 1] = c << 20 | res << 8 | (lut >> 8) << 3 | kind;
+  }
+}
+
+// A block barrier after the warp's last entry (an entry of its own when that
+// one has a barrier already, or there is none).
+void addBarrier(std::vector<ProgEntry> &es) {
+  if (es.empty() || (es.back().w[1] & kProgBarrier)) {
+    ProgEntry e;
+    e.id = 0;
+    for (uint32_t l = 0; l < 32; ++l) {
+      e.w[2 * l] = 0;
+      e.w[2 * l + 1] = kProgUnit;
+    }
+    es.push_back(e);
+  }
+  for (uint32_t l = 0; l < 32; ++l) es.back().w[2 * l + 1] |= kProgBarrier;
+}
+
 }  // namespace
 
 void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32_t G,
@@ -750,6 +806,7 @@ void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32
     std::vector<uint32_t> readersMask(pd.vpSlots + 64, 0);  // warps that read since the barrier
     std::vector<uint32_t> touched;
     uint32_t blocks = 0;
+    std::vector<std::vector<ProgEntry>> progW(so.program ? NW : 0u);  // the partition's entries per warp
     for (uint32_t lv = 0; lv < nLv;) {
       Plan plan;
       double mk = planLevel(lv, plan);
@@ -821,6 +878,19 @@ void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32
           }
         }
       out.levels++;
+      out.fusedLevels += n - 1;
+      if (so.program) {
+        if (need && blocks)
+          for (auto &e : progW) addBarrier(e);
+        for (uint32_t w = 0; w < NW; ++w)
+          for (const Unit &un : plan[w]) {
+            progW[w].push_back({});
+            encodeEntry(img.net.data(), levels[un.lv][un.i], un.g0, un.gn, so.spw, progW[w].back());
+          }
+        ++blocks;
+        lv += n;
+        continue;
+      }
       // level block: [flags][NW + 1 prefix offsets][unit offsets][pad][micro-partitions in warp order]
       while (sw.size() % 4) sw.push_back(0);
       const uint32_t blk = uint32_t(sw.size());
@@ -855,17 +925,28 @@ void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32
       out.levelDesc.push_back(blk);
       out.levelDesc.push_back(words);
       out.maxLevelWords = std::max(out.maxLevelWords, words);
-      out.fusedLevels += n - 1;
       ++blocks;
       lv += n;
     }
     pd.nLevels = blocks;  // exec-level blocks the kernel runs
+    for (const auto &es : progW) {
+      out.progBegin.push_back(uint32_t(out.progId.size()));
+      out.progBegin.push_back(uint32_t(es.size()));
+      for (const ProgEntry &e : es) {
+        out.prog.insert(out.prog.end(), e.w, e.w + 64);
+        out.progId.push_back(e.id);
+      }
+    }
     // L0 and last level scale with their op counts spread over the block
     total += double(pd.l0Count + pd.copySlots + 8 * pd.memWCount) / double(32 * NW) + 1.0;
     out.partCost[pid] = total;
   }
   while (sw.size() % 4 || sw.empty()) sw.push_back(0);
   if (out.levelDesc.empty()) out.levelDesc.assign(2, 0);
+  if (so.program) {
+    out.prog.resize(out.prog.size() + 64 * (kProgAhead + 1), 0u);  // entries are read ahead past the last one
+    out.progId.resize(out.progId.size() + 1, 0u);
+  }
 
   // items (partition, group block) onto blocks, per region, LPT by cost
   out.items.clear();

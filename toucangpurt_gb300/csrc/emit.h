@@ -56,6 +56,9 @@ struct Schedule {
   std::vector<uint32_t> words;
   std::vector<uint32_t> levelDesc;
   uint32_t maxLevelWords = 0;
+  // warp programs (SchedOpts::program): entries of 64 words, (first entry,
+  // entries) per partition and warp, micro-partition id per entry
+  std::vector<uint32_t> prog, progBegin, progId;
   std::vector<uint32_t> items;      // (part | groupBlock << 20) per region and block
   std::vector<uint32_t> itemBegin;  // [2][nBlocks + 1]
   std::vector<double> partCost;
@@ -72,6 +75,8 @@ struct Schedule {
 struct SchedOpts {
   uint32_t unitLanes = 32;       // LUTs a warp takes per unit of its level plan: 32, 64 or 128
   uint32_t levelsPerBarrier = 1;  // exec levels one block may merge: 1, 2 or 4
+  bool program = false;           // emit warp programs instead of level blocks
+  uint32_t spw = 8;               // streams per word (warp programs: one stream reads the table for every op)
 };
 
 // Word-wide evaluation of palette LUT ops.  A LUT op reads table entry

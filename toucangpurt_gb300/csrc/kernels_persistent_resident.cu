@@ -4,6 +4,6 @@
 
 namespace tgs {
 
-void *cycleKernelResident(int spw, int G) { return cycleKernelPtrT<true>(spw, G); }
+void *cycleKernelResident(int spw, int G) { return cycleKernelPtrT<kLevelsResident>(spw, G); }
 
 }  // namespace tgs

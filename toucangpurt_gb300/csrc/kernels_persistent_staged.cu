@@ -4,6 +4,6 @@
 
 namespace tgs {
 
-void *cycleKernelStaged(int spw, int G) { return cycleKernelPtrT<false>(spw, G); }
+void *cycleKernelStaged(int spw, int G) { return cycleKernelPtrT<kLevelsStaged>(spw, G); }
 
 }  // namespace tgs

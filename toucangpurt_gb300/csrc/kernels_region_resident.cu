@@ -4,6 +4,6 @@
 
 namespace tgs {
 
-void *regionKernelResident(int spw, int G) { return regionKernelPtrT<true>(spw, G); }
+void *regionKernelResident(int spw, int G) { return regionKernelPtrT<kLevelsResident>(spw, G); }
 
 }  // namespace tgs

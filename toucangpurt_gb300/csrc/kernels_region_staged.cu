@@ -4,6 +4,6 @@
 
 namespace tgs {
 
-void *regionKernelStaged(int spw, int G) { return regionKernelPtrT<false>(spw, G); }
+void *regionKernelStaged(int spw, int G) { return regionKernelPtrT<kLevelsStaged>(spw, G); }
 
 }  // namespace tgs

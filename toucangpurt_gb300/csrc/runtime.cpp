@@ -95,10 +95,12 @@ struct tgs_sim {
   // launch configuration
   tgs::LaunchCfg lc;
   uint32_t spw = 1, groups = 1, gpad = 1, nStreams = 1, regSlots = 4, exgSlots = 4, stageWords = 0;
+  uint32_t regionItems = 0;  // items of the larger region
   uint32_t resWords = 0;  // words of a block's resident exec levels (0: staged or global)
   unsigned long long memStride = 16;
 
   // device memory
+  tgs::DBuf<uint32_t> prog, progBegin, progId;         // warp programs
   tgs::DBuf<uint32_t> itemRes, resCopy, resCopyBegin;  // resident exec levels (see configure)
   tgs::DBuf<uint32_t> net, schedW, levelDesc, items, itemBegin, regs, exg, stop, stopCycle, err, errInfo, barrier, realCycles, stimReg;
   tgs::DBuf<tgs::PartDesc> parts;
@@ -186,6 +188,9 @@ void fillParams(tgs_sim *h) {
   std::memset(&p, 0, sizeof(p));
   p.net = h->net.p;
   p.sched = h->schedW.p;
+  p.prog = reinterpret_cast<const uint2 *>(h->prog.p);
+  p.progBegin = reinterpret_cast<const uint2 *>(h->progBegin.p);
+  p.progId = h->progId.p;
   p.levelDesc = reinterpret_cast<const uint2 *>(h->levelDesc.p);
   p.stageWords = h->stageWords;
   p.resWords = h->resWords;
@@ -261,6 +266,11 @@ uint32_t autoWarps(const DeviceImage &img, uint32_t G, uint32_t spw) {
   return std::clamp<uint32_t>(best, 6, 16);
 }
 
+// tgs_tune_trial.staged: 0 global, 1 staged, 2 resident, 3 warp programs
+uint32_t levelSource(const tgs_sim *h) {
+  return h->lc.lv == kLevelsProgram ? 3u : h->resWords ? 2u : h->stageWords ? 1u : 0u;
+}
+
 void configure(tgs_sim *h) {
   const tgs_options &o = h->opt;
   h->nStreams = std::max<uint32_t>(1, o.n_streams);
@@ -296,13 +306,20 @@ void configure(tgs_sim *h) {
   h->lc.G = G;
   h->lc.threads = NW * 32;
   h->lc.stream = h->stream;
-  h->lc.res = false;
-  void *fn = cycleKernelFor(int(h->spw), G, false);
-  void *fnRegion = regionKernelFor(int(h->spw), G, false);
+  // warp programs by default; the other forms on request, and for pools whose
+  // slots 0..15 are taken (the design's own numbering: operands there may be
+  // immediates, which program entries read as slots)
+  const bool program = o.resident_netlist == 0 && h->img.renumbered;
+  h->lc.lv = program ? kLevelsProgram : kLevelsStaged;
+  so.program = program;
+  so.spw = h->spw;
+  void *fn = cycleKernelFor(int(h->spw), G, h->lc.lv);
+  void *fnRegion = regionKernelFor(int(h->spw), G, h->lc.lv);
   const size_t vpBytes = size_t(h->img.maxVpSlots) * size_t(G) * 4;
   const uint32_t nGB = h->gpad / uint32_t(G);
   size_t maxItems = 1;
   for (auto &r : h->design.regionPartitionIds) maxItems = std::max(maxItems, r.size() * nGB);
+  h->regionItems = uint32_t(maxItems);
 
   // schedule (greedy gate count or learned cost); exec-level blocks are
   // staged through shared memory when two of the largest fit next to the
@@ -334,12 +351,12 @@ void configure(tgs_sim *h) {
                                        " groups needs " + std::to_string(kLutTablePadded + vpBytes) +
                                        " B of shared memory; lower groups_per_item");
   // first pass to learn the largest level block (independent of the block count)
-  buildSchedule(h->design, h->img, NW, uint32_t(G), costPtr, 1, nGB, h->sched, so);
+  if (!program) buildSchedule(h->design, h->img, NW, uint32_t(G), costPtr, 1, nGB, h->sched, so);
   // Stage buffer size: the largest level, or a smaller size that still
   // stages nearly every level when it puts more blocks on an SM (levels
   // larger than the buffers are read from global memory; mixed 4M-LUT
   // design: 4 -> 5 blocks per SM, 256K -> 310K stimulus-cycles/s)
-  uint32_t stage = o.resident_netlist == 2 ? 0u : std::min<uint32_t>(h->sched.maxLevelWords, 4096u);
+  uint32_t stage = program || o.resident_netlist == 2 ? 0u : std::min<uint32_t>(h->sched.maxLevelWords, 4096u);
   if (o.stage_words) stage = std::min<uint32_t>(stage, (o.stage_words + 3u) & ~3u);
   int perSM = shape(stage);
   if (stage) {
@@ -376,8 +393,12 @@ void configure(tgs_sim *h) {
   // a quarter more items in flight (blocks on the GPU at once, up to the
   // items of a region), so more items are evaluated side by side (a single
   // stream of the 16M-LUT design, 1,024 items per region: 1,024 blocks of 4
-  // warps instead of 760 of 6, 5.6K -> 7.6K cycles/s)
-  if (!o.warps_per_block && NW > 4) {
+  // warps instead of 760 of 6, 5.6K -> 7.6K cycles/s).  Warp programs of 8
+  // streams per word keep the design's width: their warps have a group's 8
+  // lookups each to overlap, and wider blocks balance a level better (16M-LUT
+  // design x 64 streams, 30 cycles: 6 warps 14.3 ms, 4 warps 15.0 ms; one
+  // stream, 100 cycles: 4 warps 12.7 ms, 6 warps 14.4 ms)
+  if (!o.warps_per_block && NW > 4 && (!program || h->spw == 1)) {
     int perSM4 = 0;
     TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM4, fn, 128, h->lc.smem));
     if (o.blocks_per_sm) perSM4 = std::min<int>(perSM4, int(o.blocks_per_sm));
@@ -399,7 +420,7 @@ void configure(tgs_sim *h) {
   // bulk copy per level whose latency a short level cannot hide.  Chosen
   // when every block of the grid still fits on the GPU at once.
   h->resWords = 0;
-  {
+  if (!program) {
     const uint32_t B = h->lc.blocks;
     std::vector<uint32_t> itemRes(h->sched.items.size(), 0), resCopy, resBegin(2 * (B + 1), 0), at(B, 0);
     std::vector<uint32_t> placedAt(h->design.parts.size(), UINT32_MAX);
@@ -430,7 +451,7 @@ void configure(tgs_sim *h) {
     if ((want == 0 || want == 1) && words) {
       const size_t smemRes = kLutTablePadded + vpBytes + size_t(words) * 4;
       int perSMRes = 0;
-      void *fnRes = cycleKernelFor(int(h->spw), G, true), *fnRegionRes = regionKernelFor(int(h->spw), G, true);
+      void *fnRes = cycleKernelFor(int(h->spw), G, kLevelsResident), *fnRegionRes = regionKernelFor(int(h->spw), G, kLevelsResident);
       cudaFuncAttributes ra{}, rr{};
       TGS_CUDA(cudaFuncGetAttributes(&ra, fnRes));
       TGS_CUDA(cudaFuncGetAttributes(&rr, fnRegionRes));
@@ -445,7 +466,7 @@ void configure(tgs_sim *h) {
         h->resWords = words;
         h->stageWords = 0;
         h->lc.smem = smemRes;
-        h->lc.res = true;
+        h->lc.lv = kLevelsResident;
         h->itemRes.upload(itemRes, h->stream);
         h->resCopy.upload(resCopy, h->stream);
         h->resCopyBegin.upload(resBegin, h->stream);
@@ -460,6 +481,11 @@ void configure(tgs_sim *h) {
     }
   }
   h->parts.upload(h->img.parts, h->stream);
+  if (program) {
+    h->prog.upload(h->sched.prog, h->stream);
+    h->progBegin.upload(h->sched.progBegin, h->stream);
+    h->progId.upload(h->sched.progId, h->stream);
+  }
   h->schedW.upload(h->sched.words, h->stream);
   h->levelDesc.upload(h->sched.levelDesc, h->stream);
   h->items.upload(h->sched.items, h->stream);
@@ -1007,7 +1033,7 @@ int tgs_autotune(tgs_sim *h, const tgs_tune_opts *opts, tgs_tune_trial *trials, 
             if (fits && h->lc.blocks == lastBlocks) continue;  // same grid as the previous trial
             if (fits) lastBlocks = h->lc.blocks;
             tr.blocks = fits ? h->lc.blocks : 0;
-            tr.staged = !fits ? 0u : h->resWords ? 2u : h->stageWords ? 1u : 0u;
+            tr.staged = !fits ? 0u : levelSource(h);
             for (uint32_t mode = 0; mode < 2; ++mode) {
               if (!(modes & (1u << mode))) continue;
               tr.mode = mode;
@@ -1060,7 +1086,7 @@ int tgs_autotune(tgs_sim *h, const tgs_tune_opts *opts, tgs_tune_trial *trials, 
           }
           if (fits) {
             tr.blocks = h->lc.blocks;
-            tr.staged = h->resWords ? 2u : h->stageWords ? 1u : 0u;
+            tr.staged = levelSource(h);
             resetState(h);
             fillParams(h);
             runTimed(h, 0, warm, 0);
@@ -1915,6 +1941,8 @@ extern "C" int tgs_get_design_stats(const tgs_sim *h, tgs_design_stats *o) {
     o->block_barriers = h->sched.barriers;
     o->exec_levels = h->sched.levels;
     o->fused_levels = uint32_t(h->sched.fusedLevels);
+    o->program_words = uint32_t(std::min<size_t>(h->sched.prog.size(), 0xFFFFFFFFu));
+    o->region_items = h->regionItems;
     o->makespan[0] = h->sched.makespan[0];
     o->makespan[1] = h->sched.makespan[1];
     o->smem_per_block = uint32_t(h->lc.smem);

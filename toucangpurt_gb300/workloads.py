@@ -90,7 +90,8 @@ def bench_simulator(name: str, design, symbols, *, streams: int | None = None, g
     """A simulator loaded and configured the way the benchmark runs a
     workload: `streams` resident streams (default: the workload's count),
     the CUDA-graph form unless the exec levels stay resident in shared
-    memory (then one persistent launch), and for more than one stream the
+    memory or no block has more than one item of a region (then one
+    persistent launch), and for more than one stream the
     learned schedule (every micro-partition profiled for `profile_cycles`
     cycles, repeated until about `samples` (features, clock64 cycles) samples
     are collected, the cost model trained on them).  Further tgs_options
@@ -109,8 +110,12 @@ def bench_simulator(name: str, design, symbols, *, streams: int | None = None, g
     s = sim.Simulator(**{**base, **options})
     s.init(gpu, design, symbols, False, False)
     notes = {"schedule": schedule}
-    if mode == "auto" and s.design_stats().get("resident_words"):
-        s.set_options(mode=capi.MODE_PERSISTENT)  # resident levels are loaded once per run
+    st = s.design_stats()
+    if mode == "auto" and (st["resident_words"] or (st["program_words"] and st["region_items"] <= st["blocks"])):
+        # resident levels are loaded once per run; with no more than one item per block a region is one chain of
+        # levels, which a launch per region lengthens (16M-LUT design, one stream: 12.1 ms persistent, 13.1 graph;
+        # 64 streams, three items per block: 48.8 and 47.8)
+        s.set_options(mode=capi.MODE_PERSISTENT)
     if schedule == "learned":
         t0 = time.perf_counter()
         feats = s.mpart_features()
