@@ -1277,13 +1277,16 @@ __device__ __forceinline__ bool stimValue(const KParams &p, uint32_t s, uint32_t
   uint32_t lc;
   unsigned long long seed;
   if (s >= p.nStreams) return false;  // padding slot of the last group
-  if ((p.flags & kFlagStopExit) && __ldcg(p.stopCycle + s) < cycle) return false;  // frozen after its stop
+  // the slot's words do not depend on each other: they are loaded together
+  const bool stopExit = (p.flags & kFlagStopExit) != 0;
+  const uint32_t sc = stopExit ? __ldcg(p.stopCycle + s) : 0xFFFFFFFFu;
   if (p.flags & kFlagSlots) {
-    const uint32_t q = __ldcg(p.slotStream + s);
-    if (q == kNoStream || cycle >= __ldcg(p.slotRetire + s)) return false;
-    lc = cycle - __ldcg(p.slotStart + s);
+    const uint32_t q = __ldcg(p.slotStream + s), re = __ldcg(p.slotRetire + s), st = __ldcg(p.slotStart + s);
+    if (q == kNoStream || cycle >= re || sc < cycle) return false;
+    lc = cycle - st;
     seed = __ldg(p.jobSeed + q);
   } else {
+    if (sc < cycle) return false;  // frozen after its stop
     lc = cycle;
     seed = __ldg(p.streamSeed + s);
     if (p.stimTable) {
@@ -1343,14 +1346,20 @@ __device__ void applyStimulus(const KParams &p, uint32_t cycle, uint32_t gtid, u
   }
 }
 
-// A slot retires in cycle t when its stream's last cycle was t - 1: the
-// stream's length was reached, or (stop exit) it executed a stop op in t - 1.
-__device__ __forceinline__ bool retiringAt(const KParams &p, uint32_t s, uint32_t t) {
-  if (__ldcg(p.slotStream + s) == kNoStream) return false;
-  if (__ldcg(p.slotRetire + s) == t) return true;
-  if (!(p.flags & kFlagStopExit)) return false;
-  const uint32_t sc = __ldcg(p.stopCycle + s);
-  return sc != 0xFFFFFFFFu && sc + 1u == t;
+// A slot's stream and state in cycle t.  It retires in cycle t when its
+// stream's last cycle was t - 1: the stream's length was reached, or (stop
+// exit) it executed a stop op in t - 1.  The three words are loaded together.
+struct SlotState {
+  uint32_t stream, stop;  // job stream (kNoStream: idle), stop cycle
+  bool retiring;
+};
+__device__ __forceinline__ SlotState slotState(const KParams &p, uint32_t s, uint32_t t) {
+  SlotState x;
+  const uint32_t re = __ldcg(p.slotRetire + s);
+  x.stream = __ldcg(p.slotStream + s);
+  x.stop = (p.flags & kFlagStopExit) ? __ldcg(p.stopCycle + s) : 0xFFFFFFFFu;
+  x.retiring = x.stream != kNoStream && (re == t || (x.stop != 0xFFFFFFFFu && x.stop + 1u == t));
+  return x;
 }
 
 // Streams whose register digest this cycle contributes: every active stream
@@ -1358,59 +1367,83 @@ __device__ __forceinline__ bool retiringAt(const KParams &p, uint32_t s, uint32_
 __device__ __forceinline__ bool digestStream(const KParams &p, uint32_t s, uint32_t cycle) {
   if (s >= p.nStreams) return false;
   if (p.flags & kFlagSlots) {
-    if (__ldcg(p.slotStream + s) == kNoStream) return false;
-    if (retiringAt(p, s, cycle)) return true;  // the retiring stream's final register digest
+    const SlotState x = slotState(p, s, cycle);
+    if (x.stream == kNoStream) return false;
+    // a retiring stream: its final register digest; a stopped one is frozen
+    return x.retiring || ((p.flags & kFlagDigest) && !(x.stop < cycle));
   }
-  if ((p.flags & kFlagStopExit) && __ldcg(p.stopCycle + s) < cycle) return false;  // frozen
-  return !(p.flags & kFlagSlots) || (p.flags & kFlagDigest);
+  return !((p.flags & kFlagStopExit) && __ldcg(p.stopCycle + s) < cycle);
 }
 
 // Per-cycle register digest: sum over i of mix64(i << 8 | nibble), per stream.
+// A warp takes a chunk of registers of one group; the index part of the mix is
+// computed once for the 8 streams of a word (17 instead of 27 instructions a
+// value).  Chunks of 256 registers, fewer (down to one per lane) while that
+// puts more warps of the grid to work and at most 128 sums meet on a stream's
+// accumulator.  The streams' states are read by one lane each (read one after
+// another, they were 6 us of the 33 us cycle of 280 queued streams), and the
+// eight sums meet by halving exchanges, 9 shuffled values instead of 40.
 template <int SPW>
 __device__ void digestSlice(const KParams &p, uint32_t cycle) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
-  const uint32_t chunks = (p.regSlots + 255) / 256;
+  const uint32_t warps = p.nBlocks * NW;
+  uint32_t chunk = 256, chunks = (p.regSlots + 255u) / 256u;
+  while (chunk > 32u && chunks <= 64u && chunks * p.gpad < warps) {
+    chunk >>= 1;
+    chunks = (p.regSlots + chunk - 1u) / chunk;
+  }
   const uint32_t units = chunks * p.gpad;
-  for (uint32_t u = blockIdx.x * NW + warp; u < units; u += p.nBlocks * NW) {
+  for (uint32_t u = blockIdx.x * NW + warp; u < units; u += warps) {
     const uint32_t g = u % p.gpad, ch = u / p.gpad;
-    bool want[SPW];
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < SPW; ++k) {
-      want[k] = digestStream(p, g * SPW + k, cycle);
-      any |= want[k];
-    }
-    if (!any) continue;
+    const uint32_t want = __ballot_sync(kFull, lane < SPW && digestStream(p, g * SPW + lane, cycle));
+    if (want == 0u) continue;
     unsigned long long acc[SPW];
 #pragma unroll
     for (int k = 0; k < SPW; ++k) acc[k] = 0;
-    const uint32_t end = min(p.regSlots, ch * 256 + 256);
-    for (uint32_t i = ch * 256 + lane; i < end; i += 32) {
+    const uint32_t end = min(p.regSlots, ch * chunk + chunk);
+    for (uint32_t i = ch * chunk + lane; i < end; i += 32) {
       const uint32_t w = __ldcg(p.regs + size_t(i) * p.gpad + g);
+      const MixIndex mix(i);
 #pragma unroll
-      for (int k = 0; k < SPW; ++k) acc[k] += dmix64((unsigned long long)i << 8 | nib(w, k));
+      for (int k = 0; k < SPW; ++k) acc[k] += mix(nib(w, k));
     }
+    uint32_t k = 0;  // the stream whose sum the lane ends with
+    if constexpr (SPW == 8) {
 #pragma unroll
-    for (int k = 0; k < SPW; ++k) {
-      unsigned long long a = acc[k];
-      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
-      if (lane == 0 && want[k]) atomicAdd(p.digAcc + g * SPW + k, a);
+      for (int n = 4; n > 0; n >>= 1) {  // acc[0 .. 2n) -> acc[0 .. n): the lane keeps one half
+        const bool up = (lane & (4u * n)) != 0;
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+          const unsigned long long send = up ? acc[j] : acc[j + n], keep = up ? acc[j + n] : acc[j];
+          acc[j] = keep + __shfl_xor_sync(kFull, send, 4 * n);
+        }
+        k += up ? n : 0;
+      }
+    } else {
+      for (int o = 16; o >= 4; o >>= 1) acc[0] += __shfl_xor_sync(kFull, acc[0], o);
     }
+    acc[0] += __shfl_xor_sync(kFull, acc[0], 2);
+    acc[0] += __shfl_xor_sync(kFull, acc[0], 1);
+    if ((lane & 3u) == 0u && (SPW == 8 || lane == 0u) && ((want >> k) & 1u)) atomicAdd(p.digAcc + g * SPW + k, acc[0]);
   }
 }
 
 __device__ void foldDigest(const KParams &p, uint32_t cycle, uint32_t gtid, uint32_t gthreads) {
   for (uint32_t s = gtid; s < p.nStreams; s += gthreads) {
+    const unsigned long long dg = __ldcg(p.digAcc + s), roll = __ldcg(p.roll + s);
     uint32_t q = s, lc = cycle - p.cycBase;
-    if ((p.flags & kFlagStopExit) && __ldcg(p.stopCycle + s) < cycle) continue;
     if (p.flags & kFlagSlots) {
-      q = __ldcg(p.slotStream + s);
-      if (q == kNoStream || retiringAt(p, s, cycle)) continue;  // retiring: kept for the admin phase
-      lc = cycle - __ldcg(p.slotStart + s);
+      const uint32_t start = __ldcg(p.slotStart + s);
+      const SlotState x = slotState(p, s, cycle);
+      // retiring: kept for the admin phase
+      if (x.stream == kNoStream || x.retiring || x.stop < cycle) continue;
+      q = x.stream;
+      lc = cycle - start;
+    } else if ((p.flags & kFlagStopExit) && __ldcg(p.stopCycle + s) < cycle) {
+      continue;
     }
-    const unsigned long long dg = __ldcg(p.digAcc + s);
     p.digAcc[s] = 0;
-    p.roll[s] = dmix64(p.roll[s] + dg);
+    p.roll[s] = dmix64(roll + dg);
     if (p.cycDig && lc < p.cycStride) p.cycDig[size_t(q) * p.cycStride + lc] = dg;
   }
 }
@@ -1505,15 +1538,35 @@ __device__ void eventRegion0(const KParams &p, const uint32_t *bits, uint32_t cn
       atomicOr(p.retireMask + s / SPW, 15u << (4 * (s % SPW)));
     }
   }
+  // 1 KiB of a stream's memories per warp: 16 bytes a lane and step, so that a
+  // stream of a small design spreads over the warps of the grid (a warp reading
+  // 8,192 bytes one by one took 256 dependent steps)
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
-  const uint32_t chunk = 8192, chunks = (p.memPoolSize + chunk - 1) / chunk;
+  const uint32_t chunk = 1024, chunks = (p.memPoolSize + chunk - 1) / chunk;
   const uint32_t units = cnt * chunks;
   for (uint32_t u = blockIdx.x * NW + warp; u < units; u += p.nBlocks * NW) {
-    const uint32_t s = nthRetiring(bits, nw, u / chunks), ch = u % chunks;
+    const uint32_t s = nthRetiring(bits, nw, u / chunks), at = u % chunks * chunk;
     const uint8_t *m = p.mems + s * p.memStride;
     unsigned long long a = 0;
-    const uint32_t end = min(p.memPoolSize, (ch + 1) * chunk);
-    for (uint32_t i = ch * chunk + lane; i < end; i += 32) a += dmix64((unsigned long long)i << 8 | __ldcg(m + i));
+    const uint32_t end = min(p.memPoolSize, at + chunk);
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+      const uint32_t i0 = at + 512u * h + 16u * lane;
+      if (i0 >= end) continue;
+      const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(m + i0));  // strides are whole 16-byte pieces
+      const uint32_t x[4] = {q.x, q.y, q.z, q.w}, n = min(16u, end - i0);
+      if (((q.x | q.y | q.z | q.w) & 0x80808080u) == 0u) {
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j)
+          if (j < n) a += MixIndex(i0 + j)((x[j / 4] >> (8 * (j % 4))) & 0xFFu);
+      } else {
+#pragma unroll 1
+        for (uint32_t j = 0; j < n; ++j) {
+          const uint32_t y = j < 8 ? (j < 4 ? q.x : q.y) : (j < 12 ? q.z : q.w);
+          a += dmix64((unsigned long long)(i0 + j) << 8 | ((y >> (8 * (j % 4))) & 0xFFu));
+        }
+      }
+    }
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
     if (lane == 0) atomicAdd(p.memAcc + s, a);
   }
@@ -1524,11 +1577,9 @@ __device__ void eventRegion0(const KParams &p, const uint32_t *bits, uint32_t cn
 __device__ void eventRegion1(const KParams &p, uint32_t gtid, uint32_t gthreads) {
   const uint32_t cnt = __ldcg(p.retCount);
   const uint32_t vecs = uint32_t((p.memPoolSize + 15ull) / 16);
-  const size_t total = size_t(cnt) * vecs;
-  for (size_t i = gtid; i < total; i += gthreads) {
-    const uint32_t s = __ldcg(p.retList + uint32_t(i / vecs));
-    const size_t v = i % vecs;
-    reinterpret_cast<uint4 *>(p.mems + s * p.memStride)[v] = __ldg(reinterpret_cast<const uint4 *>(p.initMems) + v);
+  for (uint32_t j = 0; j < cnt; ++j) {
+    uint4 *m = reinterpret_cast<uint4 *>(p.mems + __ldcg(p.retList + j) * p.memStride);
+    for (uint32_t v = gtid; v < vecs; v += gthreads) m[v] = __ldg(reinterpret_cast<const uint4 *>(p.initMems) + v);
   }
 }
 
@@ -1563,22 +1614,23 @@ __device__ void eventAdmit(const KParams &p, uint32_t cycle, uint32_t gtid, uint
     p.slotStart[s] = cycle + 1;
     p.slotRetire[s] = cycle + 1 + __ldg(p.jobLen + qn);
     atomicMin(p.eventHint + ((cycle + 1u) & 1u), cycle + 1 + __ldg(p.jobLen + qn));
-    // primary inputs restart from the initial register values
-    for (uint32_t inp = 0; inp < p.nStim; ++inp) {
-      const uint32_t reg = __ldg(p.stimReg + inp);
-      const uint32_t mask = (1u << __ldg(p.stimBits + inp)) - 1u;
-      const uint32_t tog = p.stimToggle ? uint32_t(__ldg(p.stimToggle + inp)) : 0u;
-      const uint32_t cur = p.initRegs[reg] & 15u;
-      uint32_t v = cur;
-      const unsigned long long h = dmix64(__ldg(p.jobSeed + qn) ^ dmix64((unsigned long long)0 << 32 | inp));
-      if (tog == 0)
-        v = uint32_t(h) & mask;
-      else
-        v = (h >> 48) < tog ? cur ^ mask : cur;
-      uint32_t *wp = p.regs + size_t(reg) * p.gpad + g;
-      atomicAnd(wp, ~(15u << (4 * k)));
-      atomicOr(wp, v << (4 * k));
-    }
+  }
+  // primary inputs restart from the initial register values: one thread per
+  // admitted stream and input (the last threads of the grid first: the first
+  // ones publish)
+  for (uint32_t x = gthreads - 1u - gtid; x < cnt * p.nStim; x += gthreads) {
+    const uint32_t j = x / p.nStim, inp = x % p.nStim;
+    if (head + j >= p.nJobs) continue;
+    const uint32_t s = __ldcg(p.retList + j), qn = __ldg(p.queueOrder + head + j), g = s / SPW, k = s % SPW;
+    const uint32_t reg = __ldg(p.stimReg + inp);
+    const uint32_t mask = (1u << __ldg(p.stimBits + inp)) - 1u;
+    const uint32_t tog = p.stimToggle ? uint32_t(__ldg(p.stimToggle + inp)) : 0u;
+    const uint32_t cur = p.initRegs[reg] & 15u;
+    const unsigned long long h = dmix64(__ldg(p.jobSeed + qn) ^ dmix64((unsigned long long)0 << 32 | inp));
+    const uint32_t v = tog == 0 ? uint32_t(h) & mask : (h >> 48) < tog ? cur ^ mask : cur;
+    uint32_t *wp = p.regs + size_t(reg) * p.gpad + g;
+    atomicAnd(wp, ~(15u << (4 * k)));
+    atomicOr(wp, v << (4 * k));
   }
   if (gtid == 0) *p.queueHead = min(head + cnt, p.nJobs);
 }
@@ -1746,7 +1798,8 @@ __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t 
     if (event) eventRegion1(p, gtid, gthreads);
     // (stop exit: applied after the region barrier, when every stop of the cycle is known)
     if ((p.flags & kFlagStimulus) && !(p.flags & kFlagStopExit) && t + 1 < cEnd) applyStimulus<SPW>(p, t + 1, gtid, gthreads);
-    if (p.flags & kFlagDigest) foldDigest(p, t, gtid, gthreads);
+    // by the last threads of the grid: the first ones write the inputs
+    if (p.flags & kFlagDigest) foldDigest(p, t, gthreads - 1u - gtid, gthreads);
   }
 }
 
