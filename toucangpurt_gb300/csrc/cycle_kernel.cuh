@@ -1648,22 +1648,30 @@ __device__ __forceinline__ bool gridSync(const KParams &p, uint32_t &gen) {
     // barrier g of the launch is complete once it reaches g * blocks, so the
     // last block to arrive has nothing more to write (wrap-safe compare)
     const uint32_t target = (gen + 1u) * gridDim.x;
-    __threadfence();
-    const uint32_t arrived = atomicAdd(p.barrier, 1u) + 1u;
-    if (arrived != target) {
-      const unsigned long long t0 = gtimer();
-      volatile uint32_t *vc = p.barrier;
-      volatile uint32_t *ve = p.err;
-      while (int32_t(*vc - target) < 0) {
-        if (*ve != 0u) { ok = 0; break; }
-        if (gtimer() - t0 > p.timeoutNs) {
-          raiseErr(p, kErrTimeout, blockIdx.x, gen + 1u, 0);
-          ok = 0;
-          break;
-        }
+    // the release orders the block's writes (the block barrier above put them
+    // before this thread's) before the arrival, the acquiring load the block's
+    // later reads after it; the error word and the time are looked at every 64
+    // polls (two full fences, the error word and the timer on every poll took
+    // 1,024 queued streams of the 4K-LUT design 39.3 ms, this 37.0)
+    uint32_t seen;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(p.barrier) : "memory");
+    ++seen;
+    unsigned long long t0 = 0;
+    for (uint32_t spin = 1; int32_t(seen - target) < 0; ++spin) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(p.barrier) : "memory");
+      if ((spin & 63u) != 0u || int32_t(seen - target) >= 0) continue;
+      if (*static_cast<volatile uint32_t *>(p.err) != 0u) {
+        ok = 0;
+        break;
+      }
+      if (t0 == 0) {
+        t0 = gtimer();
+      } else if (gtimer() - t0 > p.timeoutNs) {
+        raiseErr(p, kErrTimeout, blockIdx.x, gen + 1u, 0);
+        ok = 0;
+        break;
       }
     }
-    __threadfence();
     gen += 1u;
   }
   __syncthreads();
