@@ -914,7 +914,11 @@ __device__ __forceinline__ void runLevelsSingle(const KParams &p, const PartDesc
 
 // ---- warp programs -----------------------------------------------------------
 // A warp's part of all exec levels of a partition as one list of 256-byte
-// entries (devimage.h), read into registers kProgAhead entries early: no level
+// entries (devimage.h), read into registers kProgAhead entries early (and into
+// the L2 kProgFetch entries before that: programs larger than the L2 come from
+// HBM every cycle, whose latency two entries of a single stream do not cover:
+// 16M-LUT design, one stream, 100 cycles 12.1 -> 8.4 ms; 3, 6, 12, 24 entries
+// 8.4, 8.6, 8.7, 9.2 ms): no level
 // descriptors, unit lists, headers or staged copies are left between a level
 // barrier and the operand loads, and a warp that has less to do in a level
 // only waits at its barrier.  The staged levels spent 240 of 380 warp
@@ -951,6 +955,7 @@ __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, 
   for (uint32_t e = 0; e < begin.y; ++e) {
     const uint2 w1 = r1;
     r1 = __ldg(next);
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(next + 32u * kProgFetch));
     next += 32;
     const uint32_t kind = w.y & 3u;
     long long tm = 0;

@@ -105,7 +105,10 @@ static_assert(sizeof(PartDesc) == 96, "PartDesc size");
 //     KParams::net, (groups << 16) | (first group << 12) | bits]; groups = 0:
 //     nothing but the barrier
 enum : uint32_t { kProgTable = 0, kProgWide = 1, kProgMux = 2, kProgUnit = 3 };
-constexpr uint32_t kProgBarrier = 4u, kProgAhead = 2u;
+constexpr uint32_t kProgBarrier = 4u;
+// entries read into registers ahead of their use, and entries beyond those
+// whose lines are fetched into the L2
+constexpr uint32_t kProgAhead = 2u, kProgFetch = 4u;
 
 // Where a block reads its exec levels: staged per level into shared memory
 // (or, level by level, from global memory), resident there for the launch, or

@@ -944,7 +944,7 @@ void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32
   while (sw.size() % 4 || sw.empty()) sw.push_back(0);
   if (out.levelDesc.empty()) out.levelDesc.assign(2, 0);
   if (so.program) {
-    out.prog.resize(out.prog.size() + 64 * (kProgAhead + 1), 0u);  // entries are read ahead past the last one
+    out.prog.resize(out.prog.size() + 64 * (kProgAhead + kProgFetch + 1), 0u);  // read ahead past the last entry
     out.progId.resize(out.progId.size() + 1, 0u);
   }
 
