@@ -55,3 +55,24 @@ def test_design_numbering_keeps_other_forms(designs):
         s.init(0, dp, sp, False, False)
         st = s.design_stats()
     assert st["program_words"] == 0 and st["resident_words"] + st["stage_words"] > 0
+
+
+@pytest.mark.parametrize("blocks_per_sm", [0, 1])
+@pytest.mark.parametrize("warps", [2, 16, 17])  # 16 warps: the widest block that keeps its programs resident
+def test_persistent_programs_resident_or_streamed(designs, blocks_per_sm, warps):
+    """Persistent launches keep their programs in shared memory when every
+    block's fit (up to 8 items of a region and 512 threads) and stream them
+    otherwise; several items per block, memories, a stop design's tail lists."""
+    dp, sp, info = designs["palette"]
+    n = 8 * 40
+    cycles = np.full(n, 12, np.uint32)
+    stim = sim.StimulusSpec(7, info["pi_ids"], info["pi_bits"])
+    with sim.Simulator(n_streams=n, groups_per_item=1, blocks_per_sm=blocks_per_sm, warps_per_block=warps, mode=0) as s:
+        s.init(0, dp, sp, False, False)
+        st = s.design_stats()
+        got = s.batch_run(cycles, stim, cycle_digests=True)
+    if blocks_per_sm:
+        assert st["region_items"] > st["blocks"]  # several items of a region per block
+    ref = pyoracle.OracleDesign(dp, sp).run(cycles, stim, cycle_digests=True)
+    np.testing.assert_array_equal(got.cycle_digest, ref["cycle_digest"])
+    np.testing.assert_array_equal(got.final_mem_digest, ref["final_mem_digest"])

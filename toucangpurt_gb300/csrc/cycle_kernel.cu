@@ -271,9 +271,10 @@ __global__ void peekRegsKernel(const uint32_t *__restrict__ regs, uint32_t gpad,
 }  // namespace
 
 void *cycleKernelFor(int spw, int G, int lv) {
-  return lv == kLevelsProgram    ? cycleKernelProgram(spw, G)
-         : lv == kLevelsResident ? cycleKernelResident(spw, G)
-                                 : cycleKernelStaged(spw, G);
+  return lv == kLevelsProgramResident ? cycleKernelProgramResident(spw, G)
+         : lv == kLevelsProgram       ? cycleKernelProgram(spw, G)
+         : lv == kLevelsResident      ? cycleKernelResident(spw, G)
+                                      : cycleKernelStaged(spw, G);
 }
 
 cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n) {

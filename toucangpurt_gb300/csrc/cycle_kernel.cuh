@@ -945,18 +945,26 @@ __device__ __forceinline__ ProgOps decodeEntry(uint2 w, uint32_t vp) {
   return o;
 }
 
-template <int SPW, int G, bool PROF>
+// SH: the partition's image is in shared memory at img (entries and unit
+// records are read there), else the program is read from global memory.
+template <int SPW, int G, bool PROF, bool SH>
 __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, uint2 begin, uint2 r0, uint2 r1,
-                                           uint32_t vp, uint32_t tab, uint32_t lane, uint32_t gb) {
+                                           uint32_t img, uint32_t vp, uint32_t tab, uint32_t lane, uint32_t gb) {
   constexpr int H = G > 4 ? 4 : G;
-  const uint2 *next = p.prog + size_t(begin.x + kProgAhead) * 32u + lane;
+  const uint2 *next = SH ? nullptr : p.prog + size_t(begin.x + kProgAhead) * 32u + lane;
+  uint32_t nextS = img + 4u * begin.x + 256u * kProgAhead + 8u * lane;
   ProgOps o = decodeEntry<G>(r0, vp);
   uint2 w = r0;
   for (uint32_t e = 0; e < begin.y; ++e) {
     const uint2 w1 = r1;
-    r1 = __ldg(next);
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(next + 32u * kProgFetch));
-    next += 32;
+    if constexpr (SH) {
+      r1 = ldsV2(nextS);
+      nextS += 256u;
+    } else {
+      r1 = __ldg(next);
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(next + 32u * kProgFetch));
+      next += 32;
+    }
     const uint32_t kind = w.y & 3u;
     long long tm = 0;
     if constexpr (PROF) tm = clock64();
@@ -994,8 +1002,8 @@ __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, 
     } else {
       gn = (w.y >> 16) & 15u;
       if (gn) {
-        const Words<false> mp{p.net + w.x, 0u};
-        runRecord<SPW, G, false>(p, d, mp, mp[0], (w.y >> 12) & 15u, gn, vp, tab, lane, gb);
+        const Words<SH> mp{SH ? nullptr : p.net + w.x, img + 4u * w.x};
+        runRecord<SPW, G, SH>(p, d, mp, mp[0], (w.y >> 12) & 15u, gn, vp, tab, lane, gb);
       }
     }
     __syncwarp();
@@ -1021,6 +1029,15 @@ __device__ __forceinline__ PartDesc loadPart(const PartDesc *pd) {
   uint4 *dst = reinterpret_cast<uint4 *>(&d);
 #pragma unroll
   for (int i = 0; i < int(sizeof(PartDesc) / 16); ++i) dst[i] = __ldg(src + i);
+  return d;
+}
+
+// The same from a partition image in shared memory.
+__device__ __forceinline__ PartDesc loadPartShared(uint32_t img) {
+  PartDesc d;
+  uint4 *dst = reinterpret_cast<uint4 *>(&d);
+#pragma unroll
+  for (int i = 0; i < int(sizeof(PartDesc) / 16); ++i) dst[i] = ldsV4(img + 16u * i);
   return d;
 }
 
@@ -1054,14 +1071,20 @@ template <int SPW, int G, int LV>
 __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t tab, Stage &st, uint32_t cycle,
                          const uint32_t *retire, uint32_t res, uint32_t &resState) {
   const uint32_t pid = item & 0xFFFFFu, gb = item >> 20;
+  constexpr bool RES = LV == kLevelsResident, PRES = LV == kLevelsProgramResident, PROG = LV == kLevelsProgram || PRES;
   // read-only loads: the descriptor stays valid across the shared-memory
   // stores (whose memory clobber would otherwise force global reloads)
-  const PartDesc d = loadPart(p.parts + pid);
+  const PartDesc d = PRES ? loadPartShared(res) : loadPart(p.parts + pid);
+  // word `off` of the partition's lists
+  auto word = [&](uint32_t off) { return PRES ? ldsU32(res + 4u * off) : __ldg(p.net + off); };
   const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, warp = tid >> 5, NW = nthr >> 5;
-  constexpr bool RES = LV == kLevelsResident, PROG = LV == kLevelsProgram;
   // warp program: the first entries are on their way while the level-0 reads run
   uint2 begin = make_uint2(0u, 0u), r0 = begin, r1 = begin;
-  if constexpr (PROG) {
+  if constexpr (PRES) {
+    begin = ldsV2(res + 4u * (kImageDescWords + 2u * warp));
+    r0 = ldsV2(res + 4u * begin.x + 8u * lane);
+    r1 = ldsV2(res + 4u * begin.x + 256u + 8u * lane);
+  } else if constexpr (PROG) {
     begin = __ldg(p.progBegin + pid * NW + warp);
     r0 = __ldg(p.prog + size_t(begin.x) * 32u + lane);
     r1 = __ldg(p.prog + size_t(begin.x + 1u) * 32u + lane);
@@ -1082,12 +1105,10 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   // level 0: register / exchange reads (evalPartL0RegRead / ExgRead)
   {
     const uint32_t n = d.l0Count;
-    const uint32_t *src = p.net + d.l0Off;
-    const uint32_t *dst = src + n;
     const uint32_t *pool = d.l0Exchange ? p.exg : p.regs;
     for (uint32_t i = tid; i < n; i += nthr) {
-      const uint32_t s = __ldg(src + i);
-      const uint32_t r = (__ldg(dst + (i >> 1)) >> ((i & 1u) * 16)) & 0xFFFFu;
+      const uint32_t s = word(d.l0Off + i);
+      const uint32_t r = (word(d.l0Off + n + (i >> 1)) >> ((i & 1u) * 16)) & 0xFFFFu;
       copyInG<G>(vpAddr<G>(vp, r, 0), pool + size_t(s) * p.gpad + gb * G);
     }
   }
@@ -1104,10 +1125,10 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   // exec levels: warp w runs the units the schedule gave it
   bool levelsDone = PROG;
   if constexpr (PROG) {
-    if (p.flags & kFlagProfileMP)
-      runProgram<SPW, G, true>(p, d, begin, r0, r1, vp, tab, lane, gb);
+    if (!PRES && (p.flags & kFlagProfileMP))
+      runProgram<SPW, G, !PRES, PRES>(p, d, begin, r0, r1, res, vp, tab, lane, gb);
     else
-      runProgram<SPW, G, false>(p, d, begin, r0, r1, vp, tab, lane, gb);
+      runProgram<SPW, G, false, PRES>(p, d, begin, r0, r1, res, vp, tab, lane, gb);
   }
   if constexpr (G == 1 && RES) {
     if (res && !(p.flags & kFlagProfileMP)) {
@@ -1155,7 +1176,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   if (p.probeBuf)
     for (uint32_t i = tid; i < d.probeCount * G; i += nthr) {
       const uint32_t pi = i / G, g = i % G;
-      const uint32_t slot = __ldg(p.net + d.probeOff + 2 * pi), idx = __ldg(p.net + d.probeOff + 2 * pi + 1);
+      const uint32_t slot = word(d.probeOff + 2 * pi), idx = word(d.probeOff + 2 * pi + 1);
       p.probeBuf[size_t(idx) * p.gpad + gb * G + g] = ldsU32(vpAddr<G>(vp, slot, g));
     }
 
@@ -1208,8 +1229,8 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   if (d.copyKind != 2) {
     for (uint32_t i = tid; i < d.memWCount * G; i += nthr) {
       const uint32_t opi = i / G, g = i % G;
-      const uint32_t *r = p.net + d.memWOff + 4 * opi;
-      const uint32_t lo = __ldg(r), hi = __ldg(r + 1), w2 = __ldg(r + 2), en = __ldg(r + 3);
+      const uint32_t r = d.memWOff + 4 * opi;
+      const uint32_t lo = word(r), hi = word(r + 1), w2 = word(r + 2), en = word(r + 3);
       const unsigned long long memBase = (unsigned long long)lo | ((unsigned long long)(hi & 0x7FFFFFFFu) << 32);
       const bool multi = (hi >> 31) != 0;
       const uint32_t av = w2 & 0xFFFFu, dat = w2 >> 16;
@@ -1236,7 +1257,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
     }
     if (p.enablePrint) {
       for (uint32_t i = tid; i < d.printCount * G; i += nthr) {
-        const uint32_t w = __ldg(p.net + d.printOff + i / G), g = i % G;
+        const uint32_t w = word(d.printOff + i / G), g = i % G;
         const uint32_t en = w & 0xFFFFu, msg = w >> 16;
         const uint32_t EN = (en < 16 ? rep8(en) : ldsU32(vpAddr<G>(vp, en, g))) & ~xm[g];
         for (int k = 0; k < SPW; ++k) {
@@ -1247,7 +1268,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
     }
     for (uint32_t i = tid; i < d.stopCount * G; i += nthr) {
       const uint32_t opi = i / G, g = i % G;
-      const uint32_t sw = __ldg(p.net + d.stopOff + opi), en = sw & 0xFFFFu;
+      const uint32_t sw = word(d.stopOff + opi), en = sw & 0xFFFFu;
       const uint32_t EN = (en < 16 ? rep8(en) : ldsU32(vpAddr<G>(vp, en, g))) & ~xm[g];
       for (int k = 0; k < SPW; ++k) {
         const uint32_t s = (gb * G + g) * SPW + k;
@@ -1261,7 +1282,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
           if (p.printDiag) {
             printf("Toucan first stop: partition=%u op=%u enable_slot=%u value=%u\n", pid, opi, sw >> 16, nib(EN, k));
             for (uint32_t q = 0; q < d.printCount; ++q) {
-              const uint32_t w = __ldg(p.net + d.printOff + q);
+              const uint32_t w = word(d.printOff + q);
               if ((w & 0xFFFFu) == en && (w >> 16) < p.nPrintMsgs)
                 printf("Stop-associated message (literal): %s\n", p.printMsgs[w >> 16]);
             }
@@ -1724,15 +1745,37 @@ struct BlockSmem {
   uint32_t vp;   // shared address of the value pool
   uint32_t res;  // shared address of the resident exec levels
   uint32_t resState;  // see evalItem
+  uint32_t items;     // shared address of the block's item lists (resident programs)
   Stage st;
 };
+
+// Item list of one region (resident programs): items, then (item, shared
+// address of its partition's image) each.
+constexpr uint32_t kItemListWords = 1u + 2u * kResidentItems;
+
+__device__ __forceinline__ void loadItemLists(const KParams &p, BlockSmem &b, uint32_t *lists) {
+  b.items = uint32_t(__cvta_generic_to_shared(lists));
+  if (threadIdx.x < 2u) {
+    const uint32_t r = threadIdx.x;
+    const uint32_t *ib = p.itemBegin + r * (p.nBlocks + 1);
+    const uint32_t i0 = __ldg(ib + blockIdx.x), n = min(__ldg(ib + blockIdx.x + 1) - i0, kResidentItems);
+    uint32_t *l = lists + r * kItemListWords;
+    l[0] = n;
+    for (uint32_t i = 0; i < n; ++i) {
+      l[1 + 2 * i] = __ldg(p.items + i0 + i);
+      l[2 + 2 * i] = b.res + 4u * __ldg(p.itemRes + i0 + i);
+    }
+  }
+  __syncthreads();
+}
 
 // region: the region whose resident levels are loaded (-1: both, for the
 // persistent form).  With resident levels, stage mbarrier 0 (no stage
 // buffers then) completes their copies.
-template <int G, bool RES>
+template <int G, int LV>
 __device__ __forceinline__ bool setupBlock(const KParams &p, uint8_t *smem, unsigned long long *stageMbar, BlockSmem &b,
                                            int region) {
+  constexpr bool PRES = LV == kLevelsProgramResident, RES = LV == kLevelsResident || PRES;
   const uint32_t base = uint32_t(__cvta_generic_to_shared(smem));
   b.tab = base;
   b.st.buf0 = base + kLutTablePadded;
@@ -1773,12 +1816,17 @@ __device__ __forceinline__ bool setupBlock(const KParams &p, uint8_t *smem, unsi
             const uint32_t dst = b.res + 4u * __ldg(p.resCopy + 3 * c + 2);
             asm volatile(
                 "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                "l"(p.sched + src), "r"(4u * words), "r"(b.st.mb0)
+                "l"(p.resSrc + src), "r"(4u * words), "r"(b.st.mb0)
                 : "memory");
           }
         }
       }
     }
+  }
+  // images are read from the first item on (exec levels: after its L0 reads)
+  if (PRES && b.resState == 1u) {
+    if (!residentWait(p, b.st.mb0)) return false;
+    b.resState = 2;
   }
   return staged;
 }
@@ -1790,12 +1838,20 @@ template <int SPW, int G, int LV>
 __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t r, bool event, const uint32_t *retBits,
                            uint32_t retCnt, uint32_t cEnd, uint32_t c0) {
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
+  constexpr bool PRES = LV == kLevelsProgramResident;
   const uint32_t *ib = p.itemBegin + r * (p.nBlocks + 1);
-  const uint32_t i0 = __ldg(ib + blockIdx.x), i1 = __ldg(ib + blockIdx.x + 1);
+  const uint32_t i0 = PRES ? 0u : __ldg(ib + blockIdx.x);
+  const uint32_t i1 = PRES ? ldsU32(b.items + 4u * r * kItemListWords) : __ldg(ib + blockIdx.x + 1);
   for (uint32_t i = i0; i < i1; ++i) {
     const long long tk = clock64();
-    const uint32_t item = __ldg(p.items + i);
-    const uint32_t res = LV == kLevelsResident && p.resWords ? b.res + 4u * __ldg(p.itemRes + i) : 0u;
+    uint32_t item, res = 0u;
+    if constexpr (PRES) {
+      item = ldsU32(b.items + 4u * (r * kItemListWords + 1u + 2u * i));
+      res = ldsU32(b.items + 4u * (r * kItemListWords + 2u + 2u * i));
+    } else {
+      item = __ldg(p.items + i);
+      if (LV == kLevelsResident && p.resWords) res = b.res + 4u * __ldg(p.itemRes + i);
+    }
     evalItem<SPW, G, LV>(p, item, b.vp, b.tab, b.st, t, (event && r == 1) ? p.retireMask : nullptr, res, b.resState);
     // per-partition clock64 profile (SimEval.cu:894-983): running mean of the
     // useful ticks over cycles [100, 200) of a launch, group block 0
@@ -1822,12 +1878,16 @@ __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t 
 // queued stream retired or, resident streams with stop exit, every stream
 // stopped.
 template <int SPW, int G, int LV>
-__global__ void __launch_bounds__(1024) cycleKernel(const KParams p, uint32_t c0, uint32_t nCycles) {
+__global__ void __launch_bounds__(LV == kLevelsProgramResident ? kResidentThreads : 1024) cycleKernel(const KParams p, uint32_t c0, uint32_t nCycles) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) unsigned long long stageMbar[2];
   __shared__ uint32_t retBits[kMaxSlotWords];
   BlockSmem b;
-  if (!setupBlock<G, LV == kLevelsResident>(p, smem, stageMbar, b, -1)) return;
+  if (!setupBlock<G, LV>(p, smem, stageMbar, b, -1)) return;
+  if constexpr (LV == kLevelsProgramResident) {
+    __shared__ uint32_t itemLists[2 * kItemListWords];
+    loadItemLists(p, b, itemLists);
+  }
   const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
   const uint32_t cEnd = c0 + nCycles;
   uint32_t gen = 0;
@@ -1891,7 +1951,7 @@ __global__ void __launch_bounds__(1024) regionKernel(const KParams p, uint32_t k
   // admission words, loaded before the block setup hides their latency
   const uint32_t adm = !slots ? 0u : r == 0 ? __ldcg(p.eventHint + (t & 1u)) : __ldcg(p.retCount);
   BlockSmem b;
-  if (!setupBlock<G, LV == kLevelsResident>(p, smem, stageMbar, b, int(r))) return;
+  if (!setupBlock<G, LV>(p, smem, stageMbar, b, int(r))) return;
   uint32_t retCnt = adm;
   if (slots && r == 0) {
     retCnt = 0;

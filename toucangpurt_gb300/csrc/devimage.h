@@ -110,10 +110,23 @@ constexpr uint32_t kProgBarrier = 4u;
 // whose lines are fetched into the L2
 constexpr uint32_t kProgAhead = 2u, kProgFetch = 4u;
 
+// Partition images, the form in which a persistent launch keeps warp programs
+// in shared memory: [PartDesc, its offsets relative to the image][per warp:
+// word offset of the first entry, entries][L0 lists][memory writes][prints]
+// [stops][probes][records of the units][entries, warp after warp]; the first
+// word of a unit entry is its record's word offset in the image.
+constexpr uint32_t kImageDescWords = 24u;
+// Threads of a block of that form, at most: latency-bound launches of few
+// blocks, which take 128 registers a thread instead of 64 with spills (4K-LUT
+// design, one stream, 1,000 cycles 6.4 -> 5.7 ms; 1M-LUT design, one stream,
+// 300 cycles 5.1 -> 4.4 ms).
+constexpr uint32_t kResidentThreads = 512u;
+constexpr uint32_t kResidentItems = 8u;  // items of a region per block, at most, whose partitions stay resident
+
 // Where a block reads its exec levels: staged per level into shared memory
-// (or, level by level, from global memory), resident there for the launch, or
-// warp programs.
-enum : int { kLevelsStaged = 0, kLevelsResident = 1, kLevelsProgram = 2 };
+// (or, level by level, from global memory), resident there for the launch,
+// warp programs, or warp programs resident there for the launch.
+enum : int { kLevelsStaged = 0, kLevelsResident = 1, kLevelsProgram = 2, kLevelsProgramResident = 3 };
 
 // Kernel parameters (passed by value).
 struct KParams {
@@ -127,7 +140,8 @@ struct KParams {
   uint32_t constSlots;        // 1: value-pool slots 0..15 are free (renumbered pools) and hold the immediates
   uint32_t resWords;          // words of a block's resident exec levels (0: staged or read from global memory)
   const uint32_t *itemRes;    // per item: word offset of its partition's levels in the block's resident area
-  const uint32_t *resCopy;    // (schedule word, words, resident word) per copy: a partition's levels, contiguous
+  const uint32_t *resSrc;     // what is kept resident: exec-level blocks or partition images
+  const uint32_t *resCopy;    // (source word, words, resident word) per copy: a partition's levels, contiguous
   const uint32_t *resCopyBegin;  // [2][nBlocks + 1] prefix offsets into resCopy (triples) per region and block
   const PartDesc *parts;
   const uint8_t *constVec;

@@ -627,6 +627,13 @@ struct Dsu {
   void join(uint32_t a, uint32_t b) { p[find(a)] = find(b); }
 };
 
+// Words of a partition's lists in its image, each list padded to 4 words.
+uint32_t listWords(const PartDesc &d) {
+  auto pad = [](uint32_t n) { return (n + 3u) & ~3u; };
+  return pad(d.l0Count + (d.l0Count + 1u) / 2u) + pad(4u * d.memWCount) + pad(d.printCount) + pad(d.stopCount) +
+         pad(2u * d.probeCount);
+}
+
 // One entry of a warp program (devimage.h).
 struct ProgEntry {
   uint32_t w[64];
@@ -929,6 +936,21 @@ void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32
       lv += n;
     }
     pd.nLevels = blocks;  // exec-level blocks the kernel runs
+    if (so.program) {
+      size_t n = kImageDescWords + ((2 * NW + 3) & ~3u) + listWords(pd);
+      std::vector<uint32_t> units;
+      for (const auto &es : progW) {
+        n += 64 * es.size();
+        for (const ProgEntry &e : es)
+          if ((e.w[1] & 3u) == kProgUnit && (e.w[1] >> 16)) units.push_back(e.w[0]);
+      }
+      std::sort(units.begin(), units.end());
+      units.erase(std::unique(units.begin(), units.end()), units.end());
+      for (const auto &lvl : levels)
+        for (const MPartRef &r : lvl)
+          if (std::binary_search(units.begin(), units.end(), r.off)) n += r.words;
+      out.imageWords.push_back(uint32_t(n));
+    }
     for (const auto &es : progW) {
       out.progBegin.push_back(uint32_t(out.progId.size()));
       out.progBegin.push_back(uint32_t(es.size()));
@@ -979,6 +1001,66 @@ void buildSchedule(const SimDesignInfo &d, DeviceImage &img, uint32_t NW, uint32
     out.itemBegin[r * (nBlocks + 1) + nBlocks] = base;
   }
   if (out.items.empty()) out.items.push_back(0);
+}
+
+void buildPartImages(const DeviceImage &img, const Schedule &s, std::vector<uint32_t> &words,
+                     std::vector<uint32_t> &begin) {
+  words.clear();
+  begin.clear();
+  for (uint32_t pid = 0; pid < img.parts.size(); ++pid) {
+    const size_t base = words.size();
+    begin.push_back(uint32_t(base));
+    PartDesc d = img.parts[pid];
+    words.resize(base + kImageDescWords + 2 * s.NW, 0u);
+    auto list = [&](uint32_t &off, uint32_t n) {
+      const uint32_t at = uint32_t(words.size() - base);
+      words.insert(words.end(), img.net.begin() + off, img.net.begin() + off + n);
+      while (words.size() % 4) words.push_back(0);
+      off = at;
+    };
+    while ((words.size() - base) % 4) words.push_back(0);
+    list(d.l0Off, d.l0Count + (d.l0Count + 1) / 2);
+    list(d.memWOff, 4 * d.memWCount);
+    list(d.printOff, d.printCount);
+    list(d.stopOff, d.stopCount);
+    list(d.probeOff, 2 * d.probeCount);
+    // unit records, once each
+    std::vector<std::pair<uint32_t, uint32_t>> at;  // (offset in net, offset in the image)
+    for (const auto &lvl : img.mp[pid])
+      for (const MPartRef &r : lvl) at.push_back({r.off, r.words});
+    std::sort(at.begin(), at.end());
+    std::vector<uint32_t> placed(at.size(), UINT32_MAX);
+    const uint32_t *pb = s.progBegin.data() + 2 * size_t(pid) * s.NW;
+    auto unit = [&](uint32_t off) {
+      const size_t k = size_t(std::lower_bound(at.begin(), at.end(), std::make_pair(off, 0u)) - at.begin());
+      if (placed[k] == UINT32_MAX) {
+        placed[k] = uint32_t(words.size() - base);
+        words.insert(words.end(), img.net.begin() + off, img.net.begin() + off + at[k].second);
+      }
+      return placed[k];
+    };
+    auto isUnit = [](const uint32_t *e) { return (e[1] & 3u) == kProgUnit && (e[1] >> 16) != 0; };
+    for (uint32_t w = 0; w < s.NW; ++w)
+      for (uint32_t e = 0; e < pb[2 * w + 1]; ++e) {
+        const uint32_t *src = s.prog.data() + 64 * size_t(pb[2 * w] + e);
+        if (isUnit(src)) unit(src[0]);
+      }
+    for (uint32_t w = 0; w < s.NW; ++w) {
+      words[base + kImageDescWords + 2 * w] = uint32_t(words.size() - base);
+      words[base + kImageDescWords + 2 * w + 1] = pb[2 * w + 1];
+      for (uint32_t e = 0; e < pb[2 * w + 1]; ++e) {
+        const uint32_t *src = s.prog.data() + 64 * size_t(pb[2 * w] + e);
+        const bool u = isUnit(src);
+        const uint32_t off = u ? unit(src[0]) : 0u;
+        for (uint32_t l = 0; l < 32; ++l) {
+          words.push_back(u ? off : src[2 * l]);
+          words.push_back(src[2 * l + 1]);
+        }
+      }
+    }
+    std::memcpy(words.data() + base, &d, sizeof d);
+    if (words.size() - base != s.imageWords[pid]) throw Error(TGS_ERR_RESOURCES, "partition image not as planned");
+  }
 }
 
 }  // namespace tgs

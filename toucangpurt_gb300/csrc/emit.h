@@ -59,6 +59,8 @@ struct Schedule {
   // warp programs (SchedOpts::program): entries of 64 words, (first entry,
   // entries) per partition and warp, micro-partition id per entry
   std::vector<uint32_t> prog, progBegin, progId;
+  // words of every partition's image (devimage.h)
+  std::vector<uint32_t> imageWords;
   std::vector<uint32_t> items;      // (part | groupBlock << 20) per region and block
   std::vector<uint32_t> itemBegin;  // [2][nBlocks + 1]
   std::vector<double> partCost;
@@ -137,5 +139,9 @@ void buildSchedule(const toucanGPUSim::SimDesignInfo &d, DeviceImage &img, uint3
                    const std::vector<std::vector<std::vector<float>>> *cost, uint32_t nBlocks, uint32_t nGroupBlocks,
                    Schedule &out, const SchedOpts &so = SchedOpts());
 float gateCost(const MPartFeat &f);
+// The partition images of a schedule with warp programs, partition after
+// partition; begin: the first word of each.
+void buildPartImages(const DeviceImage &img, const Schedule &s, std::vector<uint32_t> &words,
+                     std::vector<uint32_t> &begin);
 
 }  // namespace tgs

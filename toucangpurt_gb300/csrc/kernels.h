@@ -25,6 +25,7 @@ void *cycleKernelResident(int spw, int G);
 void *regionKernelStaged(int spw, int G);
 void *regionKernelResident(int spw, int G);
 void *cycleKernelProgram(int spw, int G);
+void *cycleKernelProgramResident(int spw, int G);
 void *regionKernelProgram(int spw, int G);
 cudaError_t enqueueGraphChunk(const LaunchCfg &c, const KParams &p, uint32_t k, bool admit);
 cudaError_t launchStimulus(int spw, const KParams &p, uint32_t cycle, cudaStream_t st);

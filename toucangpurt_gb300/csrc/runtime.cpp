@@ -95,12 +95,15 @@ struct tgs_sim {
   // launch configuration
   tgs::LaunchCfg lc;
   uint32_t spw = 1, groups = 1, gpad = 1, nStreams = 1, regSlots = 4, exgSlots = 4, stageWords = 0;
+  uint32_t progResWords = 0;  // words of a block's resident partition images (0: programs read from global memory)
+  size_t progResSmem = 0;
   uint32_t regionItems = 0;  // items of the larger region
   uint32_t resWords = 0;  // words of a block's resident exec levels (0: staged or global)
   unsigned long long memStride = 16;
 
   // device memory
   tgs::DBuf<uint32_t> prog, progBegin, progId;         // warp programs
+  tgs::DBuf<uint32_t> partImages;                      // partition images (resident programs)
   tgs::DBuf<uint32_t> itemRes, resCopy, resCopyBegin;  // resident exec levels (see configure)
   tgs::DBuf<uint32_t> net, schedW, levelDesc, items, itemBegin, regs, exg, stop, stopCycle, err, errInfo, barrier, realCycles, stimReg;
   tgs::DBuf<tgs::PartDesc> parts;
@@ -194,6 +197,7 @@ void fillParams(tgs_sim *h) {
   p.levelDesc = reinterpret_cast<const uint2 *>(h->levelDesc.p);
   p.stageWords = h->stageWords;
   p.resWords = h->resWords;
+  p.resSrc = h->schedW.p;
   p.itemRes = h->itemRes.p;
   p.resCopy = h->resCopy.p;
   p.resCopyBegin = h->resCopyBegin.p;
@@ -420,10 +424,16 @@ void configure(tgs_sim *h) {
   // bulk copy per level whose latency a short level cannot hide.  Chosen
   // when every block of the grid still fits on the GPU at once.
   h->resWords = 0;
-  if (!program) {
-    const uint32_t B = h->lc.blocks;
-    std::vector<uint32_t> itemRes(h->sched.items.size(), 0), resCopy, resBegin(2 * (B + 1), 0), at(B, 0);
-    std::vector<uint32_t> placedAt(h->design.parts.size(), UINT32_MAX);
+  h->progResWords = 0;
+  // Where a block's partitions lie in its resident area: (source word, words)
+  // of each partition, one copy per block and partition.  Returns the words of
+  // the largest block.
+  const uint32_t B = h->lc.blocks;
+  std::vector<uint32_t> itemRes, resCopy, resBegin;
+  auto place = [&](auto range) {
+    itemRes.assign(h->sched.items.size(), 0);
+    resBegin.assign(2 * (B + 1), 0);
+    std::vector<uint32_t> at(B, 0), placedAt(h->design.parts.size(), UINT32_MAX);
     for (uint32_t r = 0; r < 2; ++r)
       for (uint32_t b = 0; b <= B; ++b) {
         resBegin[r * (B + 1) + b] = uint32_t(resCopy.size() / 3);
@@ -432,37 +442,78 @@ void configure(tgs_sim *h) {
         std::vector<uint32_t> placed;
         for (uint32_t i = i0; i < i1; ++i) {
           const uint32_t pid = h->sched.items[i] & 0xFFFFFu;
-          const PartDesc &pd = h->img.parts[pid];
-          if (placedAt[pid] == UINT32_MAX && pd.nLevels) {
-            const uint32_t first = h->sched.levelDesc[2 * pd.schedOff];
-            const uint32_t last = pd.schedOff + pd.nLevels - 1;
-            const uint32_t end = (h->sched.levelDesc[2 * last] + h->sched.levelDesc[2 * last + 1] + 3u) & ~3u;
-            placedAt[pid] = at[b];
-            resCopy.insert(resCopy.end(), {first, end - first, at[b]});
-            at[b] += end - first;
-            placed.push_back(pid);
+          if (placedAt[pid] == UINT32_MAX) {
+            const std::pair<uint32_t, uint32_t> w = range(pid);
+            if (w.second) {
+              placedAt[pid] = at[b];
+              resCopy.insert(resCopy.end(), {w.first, w.second, at[b]});
+              at[b] += w.second;
+              placed.push_back(pid);
+            }
           }
           itemRes[i] = placedAt[pid] == UINT32_MAX ? 0u : placedAt[pid];
         }
         for (uint32_t pid : placed) placedAt[pid] = UINT32_MAX;
       }
-    const uint32_t words = B ? *std::max_element(at.begin(), at.end()) : 0u;
+    return B ? *std::max_element(at.begin(), at.end()) : 0u;
+  };
+  // Shared memory of a resident form with `words` words kept, 0 when a block
+  // does not take it or the grid's blocks no longer fit on the GPU at once.
+  auto residentSmem = [&](int lv, bool regionToo, uint32_t words) -> size_t {
+    const size_t smemRes = kLutTablePadded + vpBytes + size_t(words) * 4;
+    void *fnRes = cycleKernelFor(int(h->spw), G, lv);
+    void *fnRegionRes = regionToo ? regionKernelFor(int(h->spw), G, lv) : nullptr;
+    cudaFuncAttributes ra{}, rr{};
+    TGS_CUDA(cudaFuncGetAttributes(&ra, fnRes));
+    if (fnRegionRes) TGS_CUDA(cudaFuncGetAttributes(&rr, fnRegionRes));
+    const size_t optinRes = size_t(h->props.sharedMemPerBlockOptin) - std::max(ra.sharedSizeBytes, rr.sharedSizeBytes);
+    if (smemRes > optinRes) return 0;
+    TGS_CUDA(cudaFuncSetAttribute(fnRes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemRes)));
+    if (fnRegionRes) TGS_CUDA(cudaFuncSetAttribute(fnRegionRes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemRes)));
+    int perSMRes = 0;
+    TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMRes, fnRes, int(h->lc.threads), smemRes));
+    if (o.blocks_per_sm) perSMRes = std::min<int>(perSMRes, int(o.blocks_per_sm));
+    return size_t(std::max(perSMRes, 0)) * h->props.multiProcessorCount >= B ? smemRes : 0;
+  };
+  // Warp programs of a persistent launch: kept in shared memory with the
+  // partitions' other constants when they fit for every block (a launch that
+  // reads them from global memory finds them in the L1 only until the next
+  // grid barrier, whose acquire empties it).  Sizes first: a program larger
+  // than the GPU's shared memory is not laid out as images at all.
+  if (program) {
+    uint32_t most = 0;
+    for (size_t k = 0; k + 1 < h->sched.itemBegin.size(); ++k)
+      if (k != B) most = std::max(most, h->sched.itemBegin[k + 1] - h->sched.itemBegin[k]);
+    // two entries are read ahead past a block's last image
+    const uint32_t words = place([&](uint32_t pid) { return std::make_pair(0u, h->sched.imageWords[pid]); }) +
+                           64u * kProgAhead;
+    const size_t smemRes = most <= kResidentItems && h->lc.threads <= kResidentThreads ? residentSmem(kLevelsProgramResident, false, words) : 0;
+    if (smemRes) {
+      std::vector<uint32_t> image, begin;
+      buildPartImages(h->img, h->sched, image, begin);
+      resCopy.clear();
+      place([&](uint32_t pid) { return std::make_pair(begin[pid], h->sched.imageWords[pid]); });
+      h->progResWords = words;
+      h->progResSmem = smemRes;
+      h->partImages.upload(image, h->stream);
+      h->itemRes.upload(itemRes, h->stream);
+      h->resCopy.upload(resCopy, h->stream);
+      h->resCopyBegin.upload(resBegin, h->stream);
+      TGS_CUDA(cudaStreamSynchronize(h->stream));  // the vectors end with this scope
+    }
+  }
+  if (!program) {
+    const uint32_t words = place([&](uint32_t pid) {
+      const PartDesc &pd = h->img.parts[pid];
+      if (!pd.nLevels) return std::make_pair(0u, 0u);
+      const uint32_t first = h->sched.levelDesc[2 * pd.schedOff];
+      const uint32_t last = pd.schedOff + pd.nLevels - 1;
+      return std::make_pair(first, ((h->sched.levelDesc[2 * last] + h->sched.levelDesc[2 * last + 1] + 3u) & ~3u) - first);
+    });
     const uint32_t want = o.resident_netlist;  // 0 auto, 1 resident, 2 global, 3 staged
     if ((want == 0 || want == 1) && words) {
-      const size_t smemRes = kLutTablePadded + vpBytes + size_t(words) * 4;
-      int perSMRes = 0;
-      void *fnRes = cycleKernelFor(int(h->spw), G, kLevelsResident), *fnRegionRes = regionKernelFor(int(h->spw), G, kLevelsResident);
-      cudaFuncAttributes ra{}, rr{};
-      TGS_CUDA(cudaFuncGetAttributes(&ra, fnRes));
-      TGS_CUDA(cudaFuncGetAttributes(&rr, fnRegionRes));
-      const size_t optinRes = size_t(h->props.sharedMemPerBlockOptin) - std::max(ra.sharedSizeBytes, rr.sharedSizeBytes);
-      if (smemRes <= optinRes) {
-        TGS_CUDA(cudaFuncSetAttribute(fnRes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemRes)));
-        TGS_CUDA(cudaFuncSetAttribute(fnRegionRes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemRes)));
-        TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMRes, fnRes, int(h->lc.threads), smemRes));
-        if (o.blocks_per_sm) perSMRes = std::min<int>(perSMRes, int(o.blocks_per_sm));
-      }
-      if (perSMRes > 0 && size_t(perSMRes) * h->props.multiProcessorCount >= B) {
+      const size_t smemRes = residentSmem(kLevelsResident, true, words);
+      if (smemRes) {
         h->resWords = words;
         h->stageWords = 0;
         h->lc.smem = smemRes;
@@ -472,7 +523,7 @@ void configure(tgs_sim *h) {
         h->resCopyBegin.upload(resBegin, h->stream);
       } else {
         if (want == 1)
-          throw Error(TGS_ERR_RESOURCES, "resident exec levels need " + std::to_string(smemRes) +
+          throw Error(TGS_ERR_RESOURCES, "resident exec levels need " + std::to_string(kLutTablePadded + vpBytes + size_t(words) * 4) +
                                              " B of shared memory per block for " + std::to_string(B) + " blocks");
         shape(stage);  // back to the staged (or global) size
       }
@@ -706,7 +757,17 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     return;
   }
   TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
-  TGS_CUDA(launchCycles(h->lc, h->kp, c0, n));
+  if (h->progResWords && !(flags & kFlagProfileMP)) {
+    LaunchCfg c = h->lc;
+    KParams p = h->kp;
+    c.lv = kLevelsProgramResident;
+    c.smem = h->progResSmem;
+    p.resWords = h->progResWords;
+    p.resSrc = h->partImages.p;
+    TGS_CUDA(launchCycles(c, p, c0, n));
+  } else {
+    TGS_CUDA(launchCycles(h->lc, h->kp, c0, n));
+  }
   h->lastLaunches = 1;
 }
 
