@@ -252,13 +252,13 @@ __global__ void scatterRegsKernel(uint32_t *__restrict__ regs, uint32_t slots, u
   }
 }
 
-// Writes nibbles (id, value) of one stream.
-__global__ void pokeRegsKernel(uint32_t *__restrict__ regs, uint32_t gpad, uint32_t g, uint32_t k,
-                               const uint32_t *__restrict__ ids, const uint8_t *__restrict__ vals, uint32_t n) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    uint32_t *w = regs + size_t(ids[i]) * gpad + g;
-    *w = (*w & ~(15u << (4 * k))) | ((uint32_t(vals[i]) & 15u) << (4 * k));
-  }
+// Writes one register's nibbles of one stream; they come as kernel arguments,
+// so that setting a register copies nothing.
+__global__ void pokeRegsKernel(uint32_t *__restrict__ regs, uint32_t gpad, uint32_t g, uint32_t k, const RegPoke q) {
+  const uint32_t i = threadIdx.x;
+  if (i >= q.n) return;
+  uint32_t *w = regs + size_t(q.id[i]) * gpad + g;
+  *w = (*w & ~(15u << (4 * k))) | ((uint32_t(q.val[i]) & 15u) << (4 * k));
 }
 
 // The nibbles of the listed register ids of one stream (readRegister).
@@ -281,6 +281,8 @@ cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint
   void *fn = cycleKernelFor(c.spw, c.G, c.lv);
   KParams pp = p;
   void *args[] = {&pp, &c0, &n};
+  // one block has no other to wait for
+  if (c.blocks == 1) return cudaLaunchKernel(fn, dim3(1), dim3(c.threads), args, c.smem, c.stream);
   return cudaLaunchCooperativeKernel(fn, dim3(c.blocks), dim3(c.threads), args, c.smem, c.stream);
 }
 
@@ -407,10 +409,9 @@ cudaError_t launchPeekRegs(const uint32_t *regs, uint32_t gpad, uint32_t g, uint
   return cudaGetLastError();
 }
 
-cudaError_t launchPokeRegs(uint32_t *regs, uint32_t gpad, uint32_t g, uint32_t k, const uint32_t *ids,
-                           const uint8_t *vals, uint32_t n, cudaStream_t st) {
-  if (!n) return cudaSuccess;
-  pokeRegsKernel<<<std::max<uint32_t>(1, std::min<uint32_t>(1024, (n + 255) / 256)), 256, 0, st>>>(regs, gpad, g, k, ids, vals, n);
+cudaError_t launchPokeRegs(uint32_t *regs, uint32_t gpad, uint32_t g, uint32_t k, const RegPoke &q, cudaStream_t st) {
+  if (!q.n) return cudaSuccess;
+  pokeRegsKernel<<<1, 32, 0, st>>>(regs, gpad, g, k, q);
   return cudaGetLastError();
 }
 

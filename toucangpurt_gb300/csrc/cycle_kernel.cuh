@@ -1935,6 +1935,18 @@ __global__ void __launch_bounds__(LV == kLevelsProgramResident ? kResidentThread
       break;
     }
   }
+  // the call's outcome for the host, which reads it after the launch instead
+  // of copying the error word and every stop flag back; every block's writes
+  // came before the last grid barrier
+  if (p.status && blockIdx.x == 0) {
+    uint32_t any = 0;
+    for (uint32_t s = threadIdx.x; s < p.nStreams; s += blockDim.x) any |= __ldcg(p.stop + s);
+    const int stopped = __syncthreads_or(int(any));
+    if (threadIdx.x == 0) {
+      p.status[1] = stopped ? 1u : 0u;
+      p.status[0] = __ldcg(p.err);
+    }
+  }
 }
 
 // Graph form: one launch per region, kernel boundaries instead of the grid

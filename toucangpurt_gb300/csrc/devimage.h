@@ -211,6 +211,8 @@ struct KParams {
   // graph form: {cycle counter, unused, end cycle, first cycle, exit} on the
   // device, so one captured chunk serves every call
   uint32_t *graphState;
+  uint32_t *status;           // page-locked host words written at the end of a persistent launch (null = off):
+                              // [0] the error word, [1] whether any stream has stopped
   uint32_t *nStopped;         // kFlagStopExit: streams stopped so far
   uint32_t *probeBuf;         // signal capture: [probe][gpad] value-pool words after the exec levels (null = off)
 };

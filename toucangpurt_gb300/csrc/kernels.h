@@ -17,6 +17,13 @@ struct LaunchCfg {
   cudaStream_t stream = nullptr;
 };
 
+// A register write: nibble val[i] to register id[i].
+struct RegPoke {
+  uint32_t n = 0;
+  uint32_t id[16];
+  uint8_t val[16];
+};
+
 void *cycleKernelFor(int spw, int G, int lv);
 void *regionKernelFor(int spw, int G, int lv);
 // instantiated one per translation unit (kernels_*.cu)
@@ -44,7 +51,6 @@ cudaError_t launchScatterRegs(uint32_t *regs, uint32_t slots, uint32_t gpad, uin
                               cudaStream_t st);
 cudaError_t launchPeekRegs(const uint32_t *regs, uint32_t gpad, uint32_t g, uint32_t k, const uint32_t *ids,
                            uint8_t *out, uint32_t n, cudaStream_t st);
-cudaError_t launchPokeRegs(uint32_t *regs, uint32_t gpad, uint32_t g, uint32_t k, const uint32_t *ids,
-                           const uint8_t *vals, uint32_t n, cudaStream_t st);
+cudaError_t launchPokeRegs(uint32_t *regs, uint32_t gpad, uint32_t g, uint32_t k, const RegPoke &q, cudaStream_t st);
 
 }  // namespace tgs

@@ -45,6 +45,9 @@ std::vector<uint8_t> readFileBytes(const std::string &path) {
   return std::vector<uint8_t>(std::istreambuf_iterator<char>(f), std::istreambuf_iterator<char>());
 }
 
+// KParams::status[0] before a launch wrote it
+constexpr uint32_t kStatusUnset = 0xFFFFFFFFu;
+
 #define TGS_CUDA(call)                                                                                     \
   do {                                                                                                     \
     cudaError_t e_ = (call);                                                                               \
@@ -88,6 +91,8 @@ struct tgs_sim {
   int device = -1;
   cudaDeviceProp props{};
   cudaStream_t stream = nullptr;
+  uint32_t *status = nullptr;   // page-locked: KParams::status
+  bool pokesInFlight = false;   // register writes launched and not waited for
   bool enablePrint = false;
   uint64_t cycleCnt = 0;
   uint64_t streamCycles = 0;  // batch bookkeeping
@@ -154,7 +159,11 @@ struct tgs_sim {
     if (device >= 0) cudaSetDevice(device);
     for (auto &g : graphs) cudaGraphExecDestroy(g.exec);
     for (auto &m : msgs) m.free();
-    if (stream) cudaStreamDestroy(stream);
+    if (stream) {
+      cudaStreamSynchronize(stream);
+      cudaStreamDestroy(stream);
+    }
+    if (status) cudaFreeHost(status);
   }
 };
 
@@ -219,6 +228,7 @@ void fillParams(tgs_sim *h) {
   p.barrier = h->barrier.p;
   p.realCycles = h->realCycles.p;
   p.nStopped = h->nStopped.p;
+  p.status = h->status;
   p.probeBuf = h->probeBuf.p;
   p.digAcc = h->digAcc.p;
   p.roll = h->roll.p;
@@ -585,6 +595,8 @@ void setupDevice(tgs_sim *h, int gpu) {
   if (!h->props.cooperativeLaunch) throw Error(TGS_ERR_NO_DEVICE, "GPU does not support cooperative launch");
   h->device = gpu;
   if (!h->stream) TGS_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+  if (!h->status) TGS_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&h->status), 2 * sizeof(uint32_t),
+                                       cudaHostAllocPortable | cudaHostAllocMapped));
 }
 
 // Probes of every signal in the symbol file (option capture_signals).
@@ -680,10 +692,16 @@ void initCommon(tgs_sim *h, int gpu, const uint8_t *design, size_t dn, const uin
   h->loaded = true;
 }
 
-void requireLoaded(tgs_sim *h) {
+// ordered: the call's own work follows the stream's (or it waits itself), so
+// register writes in flight need not be waited for.
+void requireLoaded(tgs_sim *h, bool ordered = false) {
   if (!h) throw Error(TGS_ERR_ARG, "null handle");
   if (!h->loaded) throw Error(TGS_ERR_STATE, "simulator not initialised");
   TGS_CUDA(cudaSetDevice(h->device));
+  if (!ordered && h->pokesInFlight) {
+    TGS_CUDA(cudaStreamSynchronize(h->stream));
+    h->pokesInFlight = false;
+  }
 }
 
 // Graph form: chunks of up to 32 cycles (two region launches and an admit
@@ -736,6 +754,7 @@ void runGraph(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags, uint32_t stop
 }
 
 void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
+  h->status[0] = kStatusUnset;
   if (n == 0) return;
   uint32_t stopped0 = 0;
   if (flags & kFlagStopExit) {
@@ -756,7 +775,7 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     runGraph(h, c0, n, flags, stopped0);
     return;
   }
-  TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
+  if (h->lc.blocks > 1) TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
   if (h->progResWords && !(flags & kFlagProfileMP)) {
     LaunchCfg c = h->lc;
     KParams p = h->kp;
@@ -769,6 +788,21 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     TGS_CUDA(launchCycles(h->lc, h->kp, c0, n));
   }
   h->lastLaunches = 1;
+}
+
+int stopFlag(tgs_sim *h);
+
+// Waits for the cycles just launched: errors thrown, true when any stream has
+// stopped.  A persistent launch left both in host memory; the graph form, and
+// a launch that ended before it could, leave them to be copied (three blocking
+// copies an eval() before: one cycle of the 4K-LUT design 45 -> 20 us a call;
+// setting a register, two uploads and a wait before, 17 -> 3 us).
+bool finishCycles(tgs_sim *h) {
+  TGS_CUDA(cudaStreamSynchronize(h->stream));
+  h->pokesInFlight = false;
+  if (*static_cast<volatile uint32_t *>(h->status) == kErrNone) return h->status[1] != 0u;
+  checkDeviceError(h);
+  return stopFlag(h) != 0;
 }
 
 int stopFlag(tgs_sim *h) {
@@ -797,23 +831,22 @@ void streamPos(tgs_sim *h, uint32_t s, uint32_t &g, uint32_t &k) {
 // last listed id; all nibbles written in one kernel.
 void setRegister(tgs_sim *h, uint32_t s, const char *name, uint64_t value) {
   const auto &locs = regLocs(h, name);
-  std::vector<uint32_t> ids;
-  std::vector<uint8_t> vals;
+  RegPoke q;
   uint64_t v = value;
   for (auto it = locs.rbegin(); it != locs.rend(); ++it) {
-    ids.push_back(std::get<0>(*it));
-    vals.push_back(uint8_t(v & 0xF));
+    q.id[q.n] = std::get<0>(*it);
+    q.val[q.n++] = uint8_t(v & 0xF);
     v >>= 4;
   }
   if (v != 0) throw Error(TGS_ERR_RANGE, std::string("value wider than register ") + name);
-  for (uint32_t id : ids)
-    if (id >= h->design.regPoolSize) throw Error(TGS_ERR_RANGE, "register id beyond regPool");
+  for (uint32_t i = 0; i < q.n; ++i)
+    if (q.id[i] >= h->design.regPoolSize) throw Error(TGS_ERR_RANGE, "register id beyond regPool");
   uint32_t g, k;
   streamPos(h, s, g, k);
-  h->ioIds.upload(ids, h->stream);
-  h->ioBytes.upload(vals, h->stream);
-  TGS_CUDA(launchPokeRegs(h->regs.p, h->gpad, g, k, h->ioIds.p, h->ioBytes.p, uint32_t(ids.size()), h->stream));
-  TGS_CUDA(cudaStreamSynchronize(h->stream));
+  // not waited for: the next launch follows it on the stream, and a call that
+  // looks at device memory past the stream waits first (requireLoaded)
+  TGS_CUDA(launchPokeRegs(h->regs.p, h->gpad, g, k, q, h->stream));
+  h->pokesInFlight = true;
 }
 
 // read_reg_from_gpu (SimEval.cu:1058-1069): most significant nibble first.
@@ -1199,13 +1232,12 @@ int tgs_init_from_memory(tgs_sim *h, int gpu_id, const void *design, size_t dn, 
 
 int tgs_eval(tgs_sim *h, int *stop) {
   return guard([&] {
-    requireLoaded(h);
+    requireLoaded(h, true);
     runCycles(h, uint32_t(h->cycleCnt), 1, 0);
-    TGS_CUDA(cudaStreamSynchronize(h->stream));
-    checkDeviceError(h);
+    const bool stopped = finishCycles(h);
     vcdDump(h, h->cycleCnt);  // time step = the cycle just evaluated
     h->cycleCnt += 1;
-    if (stop) *stop = stopFlag(h);
+    if (stop) *stop = stopped ? 1 : 0;
   });
 }
 
@@ -1215,11 +1247,10 @@ int tgs_eval_free_running(tgs_sim *h, uint32_t cycles, int *stop) {
     TGS_CUDA(cudaMemsetAsync(h->profU.p, 0, h->profU.n * sizeof(long long), h->stream));
     TGS_CUDA(cudaMemsetAsync(h->profT.p, 0, h->profT.n * sizeof(long long), h->stream));
     runCycles(h, uint32_t(h->cycleCnt), cycles, kFlagCountCycles | kFlagProfile);
-    TGS_CUDA(cudaStreamSynchronize(h->stream));
-    checkDeviceError(h);
+    const bool stopped = finishCycles(h);
     if (cycles) vcdDump(h, h->cycleCnt + cycles - 1);  // signals of the last cycle
     h->cycleCnt += cycles;
-    if (stop) *stop = stopFlag(h);
+    if (stop) *stop = stopped ? 1 : 0;
   });
 }
 
@@ -1240,7 +1271,7 @@ int tgs_eval_until_stop(tgs_sim *h, uint32_t max_cycles, int *stop, uint32_t *cy
 }
 
 int tgs_set_register(tgs_sim *h, const char *name, uint64_t value) {
-  return guard([&] { requireLoaded(h); setRegister(h, 0, name, value); });
+  return guard([&] { requireLoaded(h, true); setRegister(h, 0, name, value); });
 }
 int tgs_read_register(tgs_sim *h, const char *name, uint64_t *value) {
   return guard([&] {
@@ -1250,7 +1281,7 @@ int tgs_read_register(tgs_sim *h, const char *name, uint64_t *value) {
   });
 }
 int tgs_set_register_stream(tgs_sim *h, uint32_t s, const char *name, uint64_t value) {
-  return guard([&] { requireLoaded(h); setRegister(h, s, name, value); });
+  return guard([&] { requireLoaded(h, true); setRegister(h, s, name, value); });
 }
 int tgs_read_register_stream(tgs_sim *h, uint32_t s, const char *name, uint64_t *value) {
   return guard([&] {
