@@ -285,8 +285,24 @@ uint32_t levelSource(const tgs_sim *h) {
   return h->lc.lv == kLevelsProgram ? 3u : h->resWords ? 2u : h->stageWords ? 1u : 0u;
 }
 
+// Whether records of 8 and more levels hold over a quarter of the ops.
+bool chainHeavy(const DeviceImage &img) {
+  uint64_t ops = 0, deep = 0;
+  for (const auto &part : img.mp)
+    for (const auto &lv : part)
+      for (const auto &m : lv) {
+        ops += m.feat.ops;
+        if (m.feat.depth >= 8) deep += m.feat.ops;
+      }
+  return 4 * deep > ops;
+}
+
 void configure(tgs_sim *h) {
   const tgs_options &o = h->opt;
+  // warp programs by default; the other forms on request, and for pools whose
+  // slots 0..15 are taken (the design's own numbering: operands there may be
+  // immediates, which program entries read as slots)
+  const bool program = o.resident_netlist == 0 && h->img.renumbered;
   h->nStreams = std::max<uint32_t>(1, o.n_streams);
   h->spw = h->nStreams == 1 ? 1 : 8;
   h->groups = (h->nStreams + h->spw - 1) / h->spw;
@@ -296,13 +312,25 @@ void configure(tgs_sim *h) {
       G = int(o.groups_per_item);
       if (G != 1 && G != 2 && G != 4 && G != 8) throw Error(TGS_ERR_ARG, "groups_per_item must be 1, 2, 4 or 8");
     } else {
-      // default: 4 groups per item (independent work per warp) while a
-      // region still has two items per SM; fewer for few, narrow partitions
+      // default: 4 groups per item (a record's decoding is paid once for all
+      // of them) while a region has an item per SM and padding adds at most a
+      // sixth to the groups; fewer for few, narrow partitions.  Two items per
+      // SM where long middle-level chains hold a quarter of the ops (one warp
+      // runs a chain while the block waits) and for levels that are not read
+      // as warp programs.  30 cycles, ms with 1 / 2 / 4 groups per item:
+      // 1M-LUT design x 64 streams 1.66 / 1.54 / 1.36 (256 items with 4);
+      // 300K-LUT x 256 1.84 / 1.56 / 1.33 (296), x 128 1.06 / 0.91 / 1.03
+      // (148: 2 groups); 1M-LUT x 40, 5 groups, 1.26 / 1.31 / 1.36; mixed
+      // 1M-LUT design with chains x 64 5.97 / 6.71 / 7.76 (512, 256, 128).
       size_t parts = 1;
       for (auto &r : h->design.regionPartitionIds) parts = std::max(parts, r.size());
-      const size_t want = 2 * size_t(std::max(1, h->props.multiProcessorCount));
+      const size_t sms = size_t(std::max(1, h->props.multiProcessorCount));
+      const size_t want = program && !chainHeavy(h->img) ? sms : 2 * sms;
+      const bool pad = program;  // staged levels: any padding, as they were measured
       G = 4;
-      while (G > 1 && parts * ((h->groups + G - 1) / G) < want) G >>= 1;
+      while (G > 1 && (parts * ((h->groups + G - 1) / G) < want ||
+                       (pad && 6 * ((h->groups + G - 1) / G * G) > 7 * h->groups)))
+        G >>= 1;
     }
     while (G > 1 && uint32_t(G) > h->groups) G >>= 1;
   }
@@ -320,10 +348,6 @@ void configure(tgs_sim *h) {
   h->lc.G = G;
   h->lc.threads = NW * 32;
   h->lc.stream = h->stream;
-  // warp programs by default; the other forms on request, and for pools whose
-  // slots 0..15 are taken (the design's own numbering: operands there may be
-  // immediates, which program entries read as slots)
-  const bool program = o.resident_netlist == 0 && h->img.renumbered;
   h->lc.lv = program ? kLevelsProgram : kLevelsStaged;
   so.program = program;
   so.spw = h->spw;
