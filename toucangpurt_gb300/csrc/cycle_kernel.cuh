@@ -1401,14 +1401,38 @@ __device__ __forceinline__ bool digestStream(const KParams &p, uint32_t s, uint3
   return !((p.flags & kFlagStopExit) && __ldcg(p.stopCycle + s) < cycle);
 }
 
+// Sums over the warp of SPW values per lane, by halving exchanges (9 shuffled
+// values instead of 40 for 8 streams): acc[0] of the returned stream, the same
+// in every four lanes.
+template <int SPW>
+__device__ __forceinline__ uint32_t sumStreams(unsigned long long (&acc)[SPW], uint32_t lane) {
+  uint32_t k = 0;
+  if constexpr (SPW == 8) {
+#pragma unroll
+    for (int n = 4; n > 0; n >>= 1) {  // acc[0 .. 2n) -> acc[0 .. n): the lane keeps one half
+      const bool up = (lane & (4u * n)) != 0;
+#pragma unroll
+      for (int j = 0; j < n; ++j) {
+        const unsigned long long send = up ? acc[j] : acc[j + n], keep = up ? acc[j + n] : acc[j];
+        acc[j] = keep + __shfl_xor_sync(kFull, send, 4 * n);
+      }
+      k += up ? n : 0;
+    }
+  } else {
+    for (int o = 16; o >= 4; o >>= 1) acc[0] += __shfl_xor_sync(kFull, acc[0], o);
+  }
+  acc[0] += __shfl_xor_sync(kFull, acc[0], 2);
+  acc[0] += __shfl_xor_sync(kFull, acc[0], 1);
+  return k;
+}
+
 // Per-cycle register digest: sum over i of mix64(i << 8 | nibble), per stream.
 // A warp takes a chunk of registers of one group; the index part of the mix is
 // computed once for the 8 streams of a word (17 instead of 27 instructions a
 // value).  Chunks of 256 registers, fewer (down to one per lane) while that
 // puts more warps of the grid to work and at most 128 sums meet on a stream's
 // accumulator.  The streams' states are read by one lane each (read one after
-// another, they were 6 us of the 33 us cycle of 280 queued streams), and the
-// eight sums meet by halving exchanges, 9 shuffled values instead of 40.
+// another, they were 6 us of the 33 us cycle of 280 queued streams).
 template <int SPW>
 __device__ void digestSlice(const KParams &p, uint32_t cycle) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
@@ -1433,23 +1457,7 @@ __device__ void digestSlice(const KParams &p, uint32_t cycle) {
 #pragma unroll
       for (int k = 0; k < SPW; ++k) acc[k] += mix(nib(w, k));
     }
-    uint32_t k = 0;  // the stream whose sum the lane ends with
-    if constexpr (SPW == 8) {
-#pragma unroll
-      for (int n = 4; n > 0; n >>= 1) {  // acc[0 .. 2n) -> acc[0 .. n): the lane keeps one half
-        const bool up = (lane & (4u * n)) != 0;
-#pragma unroll
-        for (int j = 0; j < n; ++j) {
-          const unsigned long long send = up ? acc[j] : acc[j + n], keep = up ? acc[j + n] : acc[j];
-          acc[j] = keep + __shfl_xor_sync(kFull, send, 4 * n);
-        }
-        k += up ? n : 0;
-      }
-    } else {
-      for (int o = 16; o >= 4; o >>= 1) acc[0] += __shfl_xor_sync(kFull, acc[0], o);
-    }
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 2);
-    acc[0] += __shfl_xor_sync(kFull, acc[0], 1);
+    const uint32_t k = sumStreams(acc, lane);
     if ((lane & 3u) == 0u && (SPW == 8 || lane == 0u) && ((want >> k) & 1u)) atomicAdd(p.digAcc + g * SPW + k, acc[0]);
   }
 }

@@ -34,6 +34,9 @@ void *regionKernelResident(int spw, int G);
 void *cycleKernelProgram(int spw, int G);
 void *cycleKernelProgramResident(int spw, int G);
 void *regionKernelProgram(int spw, int G);
+// blocks that own their streams (kernels_own_streams.cu), 8 streams per word
+void *ownStreamsKernelFor(int G);
+cudaError_t launchOwnStreams(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n);
 cudaError_t enqueueGraphChunk(const LaunchCfg &c, const KParams &p, uint32_t k, bool admit);
 cudaError_t launchStimulus(int spw, const KParams &p, uint32_t cycle, cudaStream_t st);
 cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n);

@@ -102,6 +102,11 @@ struct tgs_sim {
   uint32_t spw = 1, groups = 1, gpad = 1, nStreams = 1, regSlots = 4, exgSlots = 4, stageWords = 0;
   uint32_t progResWords = 0;  // words of a block's resident partition images (0: programs read from global memory)
   size_t progResSmem = 0;
+  // blocks that own their streams: one block per group block, its items and images
+  uint32_t ownWords = 0;
+  bool ownCounts = true;  // a block's cycle counter (at most the sum of the queue's lengths) fits 32 bits
+  size_t ownSmem = 0;
+  tgs::DBuf<uint32_t> ownItems, ownBegin, ownRes, ownCopy, ownCopyBegin;
   uint32_t regionItems = 0;  // items of the larger region
   uint32_t resWords = 0;  // words of a block's resident exec levels (0: staged or global)
   unsigned long long memStride = 16;
@@ -459,6 +464,7 @@ void configure(tgs_sim *h) {
   // when every block of the grid still fits on the GPU at once.
   h->resWords = 0;
   h->progResWords = 0;
+  h->ownWords = 0;
   // Where a block's partitions lie in its resident area: (source word, words)
   // of each partition, one copy per block and partition.  Returns the words of
   // the largest block.
@@ -533,6 +539,38 @@ void configure(tgs_sim *h) {
       h->itemRes.upload(itemRes, h->stream);
       h->resCopy.upload(resCopy, h->stream);
       h->resCopyBegin.upload(resBegin, h->stream);
+      // One partition per region: blocks that own their streams, one per
+      // group block (with more partitions a group block's items are spread
+      // over several blocks instead, which the grid barrier then ties)
+      const auto &rp = h->design.regionPartitionIds;
+      if (h->spw == 8 && nGB > 1 && rp.size() == 2 && rp[0].size() == 1 && rp[1].size() == 1) {
+        const uint32_t p0 = rp[0][0], p1 = rp[1][0], w0 = h->sched.imageWords[p0], w1 = h->sched.imageWords[p1];
+        void *fnOwn = ownStreamsKernelFor(G);
+        cudaFuncAttributes oa{};
+        TGS_CUDA(cudaFuncGetAttributes(&oa, fnOwn));
+        const uint32_t ownWords = w0 + w1 + 64u * kProgAhead;
+        const size_t ownSmem = kLutTablePadded + vpBytes + size_t(ownWords) * 4;
+        if (ownSmem + oa.sharedSizeBytes <= size_t(h->props.sharedMemPerBlockOptin)) {
+          TGS_CUDA(cudaFuncSetAttribute(fnOwn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ownSmem)));
+          std::vector<uint32_t> items, ib(2 * (nGB + 1)), res, copy, cb(2 * (nGB + 1));
+          for (uint32_t r = 0; r < 2; ++r)
+            for (uint32_t b = 0; b <= nGB; ++b) {
+              ib[r * (nGB + 1) + b] = cb[r * (nGB + 1) + b] = r * nGB + b;
+              if (b == nGB) break;
+              items.push_back((r ? p1 : p0) | (b << 20));
+              res.push_back(r ? w0 : 0u);
+              copy.insert(copy.end(), {begin[r ? p1 : p0], r ? w1 : w0, r ? w0 : 0u});
+            }
+          h->ownItems.upload(items, h->stream);
+          h->ownBegin.upload(ib, h->stream);
+          h->ownRes.upload(res, h->stream);
+          h->ownCopy.upload(copy, h->stream);
+          h->ownCopyBegin.upload(cb, h->stream);
+          TGS_CUDA(cudaStreamSynchronize(h->stream));
+          h->ownWords = ownWords;
+          h->ownSmem = ownSmem;
+        }
+      }
       TGS_CUDA(cudaStreamSynchronize(h->stream));  // the vectors end with this scope
     }
   }
@@ -797,6 +835,22 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
   h->kp.flags = flags;
   if (h->opt.mode == TGS_MODE_GRAPH && !(flags & kFlagProfileMP)) {
     runGraph(h, c0, n, flags, stopped0);
+    return;
+  }
+  if (h->ownWords && h->ownCounts && !(flags & ~(kFlagStimulus | kFlagDigest | kFlagSlots | kFlagStopExit))) {
+    LaunchCfg c = h->lc;
+    KParams p = h->kp;
+    c.blocks = p.nBlocks = h->gpad / uint32_t(h->lc.G);
+    c.smem = h->ownSmem;
+    p.items = h->ownItems.p;
+    p.itemBegin = h->ownBegin.p;
+    p.itemRes = h->ownRes.p;
+    p.resCopy = h->ownCopy.p;
+    p.resCopyBegin = h->ownCopyBegin.p;
+    p.resWords = h->ownWords;
+    p.resSrc = h->partImages.p;
+    TGS_CUDA(launchOwnStreams(c, p, c0, n));
+    h->lastLaunches = 1;
     return;
   }
   if (h->lc.blocks > 1) TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
@@ -1861,7 +1915,9 @@ void batchAdmission(tgs_sim *h, const tgs_batch *job, tgs_batch_result *res, uin
     p.cycDig = h->cycDig.p;
     p.cycStride = res->cycle_stride;
   }
+  h->ownCounts = total < 0xFFFFFFF0ull;
   const float ms = runTimed(h, 0, uint32_t(last) + 1, flags | kFlagSlots);
+  h->ownCounts = true;
   h->cycleCnt = last + 1;
   if (!res) return;
   res->device_ms = ms;
