@@ -76,3 +76,28 @@ def test_persistent_programs_resident_or_streamed(designs, blocks_per_sm, warps)
     ref = pyoracle.OracleDesign(dp, sp).run(cycles, stim, cycle_digests=True)
     np.testing.assert_array_equal(got.cycle_digest, ref["cycle_digest"])
     np.testing.assert_array_equal(got.final_mem_digest, ref["final_mem_digest"])
+
+
+@pytest.mark.parametrize("name,streams", [("palette", 1500), ("mixed", 2500)])
+@pytest.mark.parametrize("groups", [1, 2, 4, 8])
+@pytest.mark.parametrize("warps", [1, 5, 8])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_teams_match_oracle(designs, name, streams, groups, warps, mode):
+    """More than one block of work per SM: teams of warps in one block per SM,
+    which look odd streams up in the nibble table; full and partial last rows
+    of teams, stops and inputs, both forms, two runs (graph chunks replayed)."""
+    dp, sp, info = designs[name]
+    n = streams if groups < 8 else 2 * streams
+    cycles = np.full(n, 5, np.uint32)
+    stim = sim.StimulusSpec(13, info["pi_ids"], info["pi_bits"])
+    with sim.Simulator(n_streams=n, groups_per_item=groups, warps_per_block=warps, mode=mode) as s:
+        s.init(0, dp, sp, False, False)
+        st = s.design_stats()
+        assert st["blocks"] > 152
+        got = s.batch_run(cycles, stim, cycle_digests=True)
+        again = s.batch_run(cycles, stim, cycle_digests=True, stop_exit=True)
+    ref = pyoracle.OracleDesign(dp, sp).run(cycles, stim, cycle_digests=True)
+    for o in (got, again):
+        np.testing.assert_array_equal(o.cycle_digest, ref["cycle_digest"])
+        np.testing.assert_array_equal(o.final_reg_digest, ref["final_reg_digest"])
+        np.testing.assert_array_equal(o.final_mem_digest, ref["final_mem_digest"])

@@ -271,10 +271,11 @@ __global__ void peekRegsKernel(const uint32_t *__restrict__ regs, uint32_t gpad,
 }  // namespace
 
 void *cycleKernelFor(int spw, int G, int lv) {
-  return lv == kLevelsProgramResident ? cycleKernelProgramResident(spw, G)
-         : lv == kLevelsProgram       ? cycleKernelProgram(spw, G)
-         : lv == kLevelsResident      ? cycleKernelResident(spw, G)
-                                      : cycleKernelStaged(spw, G);
+  return lv == kLevelsProgramTeams      ? cycleKernelProgramTeams(spw, G)
+         : lv == kLevelsProgramResident ? cycleKernelProgramResident(spw, G)
+         : lv == kLevelsProgram         ? cycleKernelProgram(spw, G)
+         : lv == kLevelsResident        ? cycleKernelResident(spw, G)
+                                        : cycleKernelStaged(spw, G);
 }
 
 cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n) {
@@ -283,13 +284,14 @@ cudaError_t launchCycles(const LaunchCfg &c, const KParams &p, uint32_t c0, uint
   void *args[] = {&pp, &c0, &n};
   // one block has no other to wait for
   if (c.blocks == 1) return cudaLaunchKernel(fn, dim3(1), dim3(c.threads), args, c.smem, c.stream);
-  return cudaLaunchCooperativeKernel(fn, dim3(c.blocks), dim3(c.threads), args, c.smem, c.stream);
+  return cudaLaunchCooperativeKernel(fn, dim3(c.blocks), dim3(c.threads, c.teams), args, c.smem, c.stream);
 }
 
 void *regionKernelFor(int spw, int G, int lv) {
-  return lv == kLevelsProgram    ? regionKernelProgram(spw, G)
-         : lv == kLevelsResident ? regionKernelResident(spw, G)
-                                 : regionKernelStaged(spw, G);
+  return lv == kLevelsProgramTeams ? regionKernelProgramTeams(spw, G)
+         : lv == kLevelsProgram    ? regionKernelProgram(spw, G)
+         : lv == kLevelsResident   ? regionKernelResident(spw, G)
+                                   : regionKernelStaged(spw, G);
 }
 
 // Enqueues one chunk of k cycles in graph form on the stream (captured by
@@ -302,7 +304,7 @@ cudaError_t enqueueGraphChunk(const LaunchCfg &c, const KParams &p, uint32_t k, 
     for (uint32_t r = 0; r < 2; ++r) {
       uint32_t ki = i, ri = r;
       void *args[] = {&pp, &ki, &ri};
-      cudaError_t e = cudaLaunchKernel(fn, dim3(c.blocks), dim3(c.threads), args, c.smem, c.stream);
+      cudaError_t e = cudaLaunchKernel(fn, dim3(c.blocks), dim3(c.threads, c.teams), args, c.smem, c.stream);
       if (e != cudaSuccess) return e;
     }
     if ((p.flags & kFlagStopExit) && (p.flags & kFlagStimulus)) {

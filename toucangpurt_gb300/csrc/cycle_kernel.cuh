@@ -165,6 +165,24 @@ __device__ __forceinline__ uint32_t vpAddr(uint32_t vp, uint32_t slot, uint32_t 
   return vp + 4u * (slot * uint32_t(G) + g);
 }
 
+// ---- teams of warps ------------------------------------------------------------
+// kLevelsProgramTeams: an SM's share of the grid is one block of several teams
+// (threadIdx.y) of blockDim.x threads, which share the tables in shared memory;
+// each team does the work of one block of the other forms, with a named barrier
+// of its own.
+template <int LV>
+__device__ __forceinline__ void teamSync() {
+  if constexpr (LV == kLevelsProgramTeams)
+    asm volatile("bar.sync %0, %1;" ::"r"(threadIdx.y + 1u), "r"(blockDim.x) : "memory");
+  else
+    __syncthreads();
+}
+// The work block: teams of one number lie one per SM, as blocks would.
+template <int LV>
+__device__ __forceinline__ uint32_t workBlock() {
+  return LV == kLevelsProgramTeams ? threadIdx.y * gridDim.x + blockIdx.x : blockIdx.x;
+}
+
 // ---- truth-table lookup ---------------------------------------------------
 // index = lutIndex + (a << 8 | b << 4 | c) per stream (SimEval.cu:353,410);
 // tab = shared address of the staged table.
@@ -205,6 +223,52 @@ __device__ __forceinline__ uint32_t lookup<8>(uint32_t tab, uint32_t base, uint3
   const uint32_t lo = __byte_perm(__byte_perm(r0, r2, 0x0040), __byte_perm(r4, r6, 0x0040), 0x5410);
   const uint32_t hi = __byte_perm(__byte_perm(r1, r3, 0x0040), __byte_perm(r5, r7, 0x0040), 0x5410);
   return lo | (hi << 4);
+}
+
+// The table a second time, for teams of warps that share a block's shared
+// memory: 8 nibbles a word, every word 32 times, once in each lane's bank
+// (kNibbleRows rows of 128 bytes after the byte table), so that a lane reads
+// its own bank whatever the index.  A byte lookup costs the shared-memory pipe
+// about 3.4 wavefronts (32 random bytes over 32 banks) and 4 ALU operations, a
+// nibble lookup 1 wavefront and 5; lookups by bytes alone are bound by the one
+// (27 pipe cycles for 8 streams of a warp), by nibbles alone by the other (24
+// measured), half of each by neither (a quarter: half the gain).  100 cycles:
+// 16M-LUT design x 64 streams 47.2 -> 43.1 ms, 1M-LUT x 64 5.0 -> 4.6, 20 cycles
+// of the mixed 4M-LUT design x 256 16.1 -> 15.4.
+__device__ __forceinline__ uint32_t ldsNibbles(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+
+// 8 streams, the even ones by bytes, the odd ones by nibbles: a permute forms
+// two 16-bit indices, one multiply-add adds lutIndex and scales both by 4
+// (bits 0..4: the nibble's place, above: the word), a rotation brings the
+// nibble to its stream's place.
+template <int SPW, bool HYB>
+__device__ __forceinline__ uint32_t lookupIn(uint32_t tab, uint32_t base, uint32_t A, uint32_t B, uint32_t C) {
+  if constexpr (!HYB) {
+    return lookup<SPW>(tab, base, A, B, C);
+  } else {
+    const uint32_t bcE = ((B & 0x0F0F0F0Fu) << 4) | (C & 0x0F0F0F0Fu);
+    const uint32_t bcO = (B & 0xF0F0F0F0u) | ((C >> 4) & 0x0F0F0F0Fu);
+    const uint32_t aE = A & 0x0F0F0F0Fu, aO = (A >> 4) & 0x0F0F0F0Fu;
+    const uint32_t t = tab + base;
+    const uint32_t r0 = ldsTab(t + prmtIdx(bcE, aE, 0xCC40u)), r2 = ldsTab(t + prmtIdx(bcE, aE, 0xDD51u));
+    const uint32_t r4 = ldsTab(t + prmtIdx(bcE, aE, 0xEE62u)), r6 = ldsTab(t + prmtIdx(bcE, aE, 0xFF73u));
+    const uint32_t col = tab + kByteTableBytes + (threadIdx.x & 31u) * 4u, base4 = base * 0x40004u;
+    uint32_t out = 0;
+    auto one = [&](uint32_t q, uint32_t k) {
+      const uint32_t w = ldsNibbles(col + ((q << 2) & 0x3FF80u));
+      out |= __funnelshift_r(w, w, q - 4u * k) & (15u << (4u * k));
+    };
+    const uint32_t q1 = __byte_perm(bcO, aO, 0x5140) * 4u + base4, q5 = __byte_perm(bcO, aO, 0x7362) * 4u + base4;
+    one(q1, 1);
+    one(q1 >> 16, 3);
+    one(q5, 5);
+    one(q5 >> 16, 7);
+    return __byte_perm(__byte_perm(r0, r2, 0x0040), __byte_perm(r4, r6, 0x0040), 0x5410) | out;
+  }
 }
 
 // ---- value-pool words of G groups ----------------------------------------
@@ -277,7 +341,7 @@ __device__ __forceinline__ void copyOutG(uint32_t *__restrict__ dst, uint32_t sr
 // multiplexer (kind 1: a ? b : c, kind 2: a ? c : b) starts from the pass-c
 // (pass-b) row and blends in the other operand where the select nibble is 1;
 // a word with a select nibble above 1 reads the table window instead.
-template <int H>
+template <int H, bool HYB = false>
 __device__ __forceinline__ void fastTop(uint32_t tab, uint32_t lut, uint32_t kind, uint32_t g, const uint32_t (&A)[H],
                                         const uint32_t (&B)[H], const uint32_t (&C)[H], uint32_t (&v)[H], bool anySel) {
   g = kind == 0u ? g : kind == 1u ? kGPassC : kGPassB;
@@ -296,7 +360,7 @@ __device__ __forceinline__ void fastTop(uint32_t tab, uint32_t lut, uint32_t kin
         const uint32_t X = kind == 1u ? B[i] : C[i];
         v[i] ^= m & (X ^ v[i]);
       } else {
-        v[i] = lookup<8>(tab, lut, A[i], B[i], C[i]);
+        v[i] = lookupIn<8, HYB>(tab, lut, A[i], B[i], C[i]);
       }
     }
   }
@@ -305,7 +369,7 @@ __device__ __forceinline__ void fastTop(uint32_t tab, uint32_t lut, uint32_t kin
 // ---- micro-partitions (evalSingleMicroPart, SimEval.cu:304-580) -----------
 // One pass of a LUT micro-partition over H stream groups starting at group
 // h0 of the item (value-pool words [slot][G]).
-template <int SPW, int G, int H, bool SH>
+template <int SPW, int G, int H, bool SH, bool HYB = false>
 __device__ __forceinline__ void evalLutPass(const Words<SH> mp, uint32_t hdr, uint32_t vp, uint32_t tab, uint32_t lane,
                                             bool constSlots, uint32_t h0) {
   const uint32_t W = (hdr >> 2) & 63u, nMid = (hdr >> 8) & 255u, nWB = (hdr >> 16) & 63u;
@@ -365,10 +429,10 @@ __device__ __forceinline__ void evalLutPass(const Words<SH> mp, uint32_t hdr, ui
       }
     }
     if (SPW == 8 && fastRec) {
-      fastTop<H>(tab, lut, kind, fg, A, B, C, v, (hdr & kMPFastSel) != 0);
+      fastTop<H, HYB>(tab, lut, kind, fg, A, B, C, v, (hdr & kMPFastSel) != 0);
     } else {
 #pragma unroll
-      for (int g = 0; g < H; ++g) v[g] = lut ? lookup<SPW>(tab, lut, A[g], B[g], C[g]) : C[g];
+      for (int g = 0; g < H; ++g) v[g] = lut ? lookupIn<SPW, HYB>(tab, lut, A[g], B[g], C[g]) : C[g];
     }
   } else {
 #pragma unroll
@@ -387,7 +451,7 @@ __device__ __forceinline__ void evalLutPass(const Words<SH> mp, uint32_t hdr, ui
       const uint32_t A = a6 < 32 ? rep8(a6) : As;
       const uint32_t B = b6 < 32 ? rep8(b6) : Bs;
       const uint32_t C = c6 < 32 ? rep8(c6) : Cs;
-      nv[g] = lut ? lookup<SPW>(tab, lut, A, B, C) : C;
+      nv[g] = lut ? lookupIn<SPW, HYB>(tab, lut, A, B, C) : C;
     }
 #pragma unroll
     for (int g = 0; g < H; ++g) v[g] = nv[g];
@@ -442,12 +506,12 @@ __device__ __forceinline__ void evalLutPass(const Words<SH> mp, uint32_t hdr, ui
 // pools never use them), so operands are loaded without a branch.  More than
 // 4 groups run as passes of 4 (the record is read once per pass from shared
 // memory; the unit's bookkeeping is paid once).
-template <int SPW, int G, bool SH>
+template <int SPW, int G, bool SH, bool HYB = false>
 __device__ __forceinline__ void evalLut(const Words<SH> mp, uint32_t hdr, uint32_t vp, uint32_t tab, uint32_t lane,
                                         bool constSlots) {
   constexpr int H = G > 4 ? 4 : G;
 #pragma unroll 1
-  for (uint32_t h0 = 0; h0 < uint32_t(G); h0 += H) evalLutPass<SPW, G, H, SH>(mp, hdr, vp, tab, lane, constSlots, h0);
+  for (uint32_t h0 = 0; h0 < uint32_t(G); h0 += H) evalLutPass<SPW, G, H, SH, HYB>(mp, hdr, vp, tab, lane, constSlots, h0);
 }
 
 // Special micro-partitions run on the stream groups [g0, g0 + gn) of the
@@ -658,11 +722,11 @@ __device__ __forceinline__ void stageCopy(const Stage &st, uint32_t b, const uin
 __device__ __forceinline__ void stageCopyWait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // A micro-partition's record for the stream groups [g0, g0 + gn) of the item.
-template <int SPW, int G, bool SH>
+template <int SPW, int G, bool SH, bool HYB = false>
 __device__ __forceinline__ void runRecord(const KParams &p, const PartDesc &d, const Words<SH> mp, uint32_t hdr,
                                           uint32_t g0, uint32_t gn, uint32_t vp, uint32_t tab, uint32_t lane,
                                           uint32_t gb) {
-  if ((hdr & 3u) == kMPLut) evalLut<SPW, G, SH>(mp, hdr, vp, tab, lane, p.constSlots != 0);  // always every group
+  if ((hdr & 3u) == kMPLut) evalLut<SPW, G, SH, HYB>(mp, hdr, vp, tab, lane, p.constSlots != 0);  // always every group
   else if ((hdr & 3u) == kMPVecRead) evalVecRead<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn);
   else if ((hdr & 3u) == kMPVecOp) evalVecOp<SPW, G, SH>(p, d, mp, hdr, vp, lane, g0, gn);
   else evalMemRead<SPW, G, SH>(p, mp, hdr, vp, lane, gb, g0, gn);
@@ -945,12 +1009,14 @@ __device__ __forceinline__ ProgOps decodeEntry(uint2 w, uint32_t vp) {
   return o;
 }
 
-// SH: the partition's image is in shared memory at img (entries and unit
-// records are read there), else the program is read from global memory.
-template <int SPW, int G, bool PROF, bool SH>
+// Resident programs: the partition's image is in shared memory at img
+// (entries and unit records are read there), else the program is read from
+// global memory.
+template <int SPW, int G, bool PROF, int LV>
 __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, uint2 begin, uint2 r0, uint2 r1,
                                            uint32_t img, uint32_t vp, uint32_t tab, uint32_t lane, uint32_t gb) {
   constexpr int H = G > 4 ? 4 : G;
+  constexpr bool SH = LV == kLevelsProgramResident, HYB = LV == kLevelsProgramTeams;
   const uint2 *next = SH ? nullptr : p.prog + size_t(begin.x + kProgAhead) * 32u + lane;
   uint32_t nextS = img + 4u * begin.x + 256u * kProgAhead + 8u * lane;
   ProgOps o = decodeEntry<G>(r0, vp);
@@ -978,7 +1044,7 @@ __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, 
         loadG<H>(o.aC + 4u * h, C);
 #pragma unroll
         for (int g = 0; g < H; ++g) {
-          const uint32_t T = lookup<SPW>(tab, o.lut, A[g], B[g], C[g]);
+          const uint32_t T = lookupIn<SPW, HYB>(tab, o.lut, A[g], B[g], C[g]);
           v[g] = o.lut ? T : C[g];
         }
         storeG<H>(o.aR + 4u * h, v);
@@ -992,9 +1058,9 @@ __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, 
           loadG<H>(o.aC + 4u * h, C);
           if (kind == kProgMux) {
             loadG<H>(o.aA + 4u * h, A);
-            fastTop<H>(tab, o.lut & 0x3FFu, o.lut >> 11, o.lut & 15u, A, B, C, v, true);
+            fastTop<H, HYB>(tab, o.lut & 0x3FFu, o.lut >> 11, o.lut & 15u, A, B, C, v, true);
           } else {
-            fastTop<H>(tab, 0u, 0u, o.lut, A, B, C, v, false);
+            fastTop<H, HYB>(tab, 0u, 0u, o.lut, A, B, C, v, false);
           }
           storeG<H>(o.aR + 4u * h, v);
         }
@@ -1003,7 +1069,7 @@ __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, 
       gn = (w.y >> 16) & 15u;
       if (gn) {
         const Words<SH> mp{SH ? nullptr : p.net + w.x, img + 4u * w.x};
-        runRecord<SPW, G, SH>(p, d, mp, mp[0], (w.y >> 12) & 15u, gn, vp, tab, lane, gb);
+        runRecord<SPW, G, SH, HYB>(p, d, mp, mp[0], (w.y >> 12) & 15u, gn, vp, tab, lane, gb);
       }
     }
     __syncwarp();
@@ -1016,7 +1082,7 @@ __device__ __forceinline__ void runProgram(const KParams &p, const PartDesc &d, 
     }
     // the next entry's addresses are ready before the barrier
     o = decodeEntry<G>(w1, vp);
-    if (w.y & kProgBarrier) __syncthreads();
+    if (w.y & kProgBarrier) teamSync<LV>();
     w = w1;
   }
 }
@@ -1071,7 +1137,7 @@ template <int SPW, int G, int LV>
 __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t tab, Stage &st, uint32_t cycle,
                          const uint32_t *retire, uint32_t res, uint32_t &resState) {
   const uint32_t pid = item & 0xFFFFFu, gb = item >> 20;
-  constexpr bool RES = LV == kLevelsResident, PRES = LV == kLevelsProgramResident, PROG = LV == kLevelsProgram || PRES;
+  constexpr bool RES = LV == kLevelsResident, PRES = LV == kLevelsProgramResident, PROG = LV == kLevelsProgram || LV == kLevelsProgramTeams || PRES;
   // read-only loads: the descriptor stays valid across the shared-memory
   // stores (whose memory clobber would otherwise force global reloads)
   const PartDesc d = PRES ? loadPartShared(res) : loadPart(p.parts + pid);
@@ -1113,7 +1179,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
     }
   }
   if (cap) stageCopyWait();  // the first level's pieces, before the barrier that publishes them
-  __syncthreads();
+  teamSync<LV>();
   // resident levels: the block's copies were issued at setup and overlapped
   // the level-0 reads; on a (never expected) timeout the levels are read from
   // global memory and the error word ends the launch
@@ -1125,10 +1191,10 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   // exec levels: warp w runs the units the schedule gave it
   bool levelsDone = PROG;
   if constexpr (PROG) {
-    if (!PRES && (p.flags & kFlagProfileMP))
-      runProgram<SPW, G, !PRES, PRES>(p, d, begin, r0, r1, res, vp, tab, lane, gb);
+    if (LV == kLevelsProgram && (p.flags & kFlagProfileMP))
+      runProgram<SPW, G, LV == kLevelsProgram, LV>(p, d, begin, r0, r1, res, vp, tab, lane, gb);
     else
-      runProgram<SPW, G, false, PRES>(p, d, begin, r0, r1, res, vp, tab, lane, gb);
+      runProgram<SPW, G, false, LV>(p, d, begin, r0, r1, res, vp, tab, lane, gb);
   }
   if constexpr (G == 1 && RES) {
     if (res && !(p.flags & kFlagProfileMP)) {
@@ -1143,7 +1209,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
     if constexpr (RES) {
       if (res) {
         const Words<true> blk{nullptr, res + 4u * (cur.x - x0)};
-        if (lv > 0 && (blk[0] & 1u)) __syncthreads();
+        if (lv > 0 && (blk[0] & 1u)) teamSync<LV>();
         runLevel<SPW, G, true>(p, d, blk, vp, tab, lane, warp, NW, gb);
         cur = nxt;
         nxt = after;
@@ -1155,13 +1221,13 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
       // the barrier, visible; the buffers are reused every second level
       if (lv > 0) {
         stageCopyWait();
-        __syncthreads();
+        teamSync<LV>();
       }
       if (lv + 1 < d.nLevels && nxt.y <= cap && warp == NW - 1)
         stageCopy(st, (lv + 1) & 1u, p.sched + nxt.x, nxt.y, lane, 32u);
       staged = cur.y <= cap;
     } else if (lv > 0 && (__ldg(p.sched + cur.x) & 1u)) {
-      __syncthreads();
+      teamSync<LV>();
     }
     if (staged)
       runLevel<SPW, G, true>(p, d, Words<true>{nullptr, st.buf0 + (lv & 1u) * st.bytes}, vp, tab, lane, warp, NW, gb);
@@ -1170,7 +1236,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
     cur = nxt;
     nxt = after;
   }
-  __syncthreads();
+  teamSync<LV>();
 
   // signal capture: the value-pool slots the symbol file names as signals
   if (p.probeBuf)
@@ -1292,7 +1358,7 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
     }
   }
   // the next item reuses the value pool
-  __syncthreads();
+  teamSync<LV>();
 }
 
 // ---- stimulus / digests ------------------------------------------------------
@@ -1434,7 +1500,7 @@ __device__ __forceinline__ uint32_t sumStreams(unsigned long long (&acc)[SPW], u
 // accumulator.  The streams' states are read by one lane each (read one after
 // another, they were 6 us of the 33 us cycle of 280 queued streams).
 template <int SPW>
-__device__ void digestSlice(const KParams &p, uint32_t cycle) {
+__device__ void digestSlice(const KParams &p, uint32_t cycle, uint32_t block) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
   const uint32_t warps = p.nBlocks * NW;
   uint32_t chunk = 256, chunks = (p.regSlots + 255u) / 256u;
@@ -1443,7 +1509,7 @@ __device__ void digestSlice(const KParams &p, uint32_t cycle) {
     chunks = (p.regSlots + chunk - 1u) / chunk;
   }
   const uint32_t units = chunks * p.gpad;
-  for (uint32_t u = blockIdx.x * NW + warp; u < units; u += warps) {
+  for (uint32_t u = block * NW + warp; u < units; u += warps) {
     const uint32_t g = u % p.gpad, ch = u / p.gpad;
     const uint32_t want = __ballot_sync(kFull, lane < SPW && digestStream(p, g * SPW + lane, cycle));
     if (want == 0u) continue;
@@ -1676,7 +1742,7 @@ __device__ __forceinline__ bool gridSync(const KParams &p, uint32_t &gen) {
   // a one-block grid (a single stream of a small design): the block barrier
   // already orders the block's global writes before its later reads
   if (gridDim.x == 1) return true;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
     ok = 1;
     // arrivals only ever add to the counter (zeroed before each launch):
     // barrier g of the launch is complete once it reaches g * blocks, so the
@@ -1717,13 +1783,13 @@ __device__ bool stageTable(const KParams &p, uint8_t *tab) {
   __shared__ __align__(8) unsigned long long mbar;
   const uint32_t mb = uint32_t(__cvta_generic_to_shared(&mbar));
   const uint32_t dst = uint32_t(__cvta_generic_to_shared(tab));
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(kLutTablePadded) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                  "l"(p.lutTable), "r"(kLutTablePadded), "r"(mb)
@@ -1791,8 +1857,10 @@ __device__ __forceinline__ bool setupBlock(const KParams &p, uint8_t *smem, unsi
   b.st.mb0 = uint32_t(__cvta_generic_to_shared(&stageMbar[0]));
   b.res = b.st.buf0 + 2u * b.st.bytes;
   b.vp = b.res + (RES ? 4u * p.resWords : 0u);
+  if constexpr (LV == kLevelsProgramTeams)
+    b.vp = base + kTeamTableBytes + threadIdx.y * (4u * G) * p.maxVpSlots;
   b.resState = 0;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && threadIdx.y == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b.st.mb0) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b.st.mb0 + 8u) : "memory");
   }
@@ -1800,6 +1868,16 @@ __device__ __forceinline__ bool setupBlock(const KParams &p, uint8_t *smem, unsi
     for (uint32_t i = threadIdx.x; i < 16u * G; i += blockDim.x) stsU32(b.vp + 4u * i, rep8(i / G));
   const bool staged = stageTable(p, smem);
   __syncthreads();
+  if constexpr (LV == kLevelsProgramTeams) {
+    // the nibble table from the byte table: a warp a row, every lane its bank
+    const uint32_t lane = threadIdx.x & 31u, warps = (blockDim.x * blockDim.y) >> 5;
+    for (uint32_t r = (threadIdx.y * blockDim.x + threadIdx.x) >> 5; r < kNibbleRows; r += warps) {
+      const uint2 q = ldsV2(b.tab + 8u * r);  // the row's 8 entries, one a byte
+      auto pack = [](uint32_t x) { return (x & 15u) | (x >> 4 & 0xF0u) | (x >> 8 & 0xF00u) | (x >> 12 & 0xF000u); };
+      stsU32(b.tab + kByteTableBytes + 128u * r + 4u * lane, pack(q.x) | pack(q.y) << 16);
+    }
+    __syncthreads();
+  }
   if (RES && p.resWords) {
     // the block's partitions: one bulk copy each, completed on mbarrier 0
     const uint32_t r0 = region < 0 ? 0u : uint32_t(region), r1 = region < 0 ? 1u : uint32_t(region);
@@ -1845,11 +1923,13 @@ __device__ __forceinline__ bool setupBlock(const KParams &p, uint8_t *smem, unsi
 template <int SPW, int G, int LV>
 __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t r, bool event, const uint32_t *retBits,
                            uint32_t retCnt, uint32_t cEnd, uint32_t c0) {
-  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
+  const uint32_t block = workBlock<LV>();
+  if (LV == kLevelsProgramTeams && block >= p.nBlocks) return;  // a team without work
+  const uint32_t gtid = block * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
   constexpr bool PRES = LV == kLevelsProgramResident;
   const uint32_t *ib = p.itemBegin + r * (p.nBlocks + 1);
-  const uint32_t i0 = PRES ? 0u : __ldg(ib + blockIdx.x);
-  const uint32_t i1 = PRES ? ldsU32(b.items + 4u * r * kItemListWords) : __ldg(ib + blockIdx.x + 1);
+  const uint32_t i0 = PRES ? 0u : __ldg(ib + block);
+  const uint32_t i1 = PRES ? ldsU32(b.items + 4u * r * kItemListWords) : __ldg(ib + block + 1);
   for (uint32_t i = i0; i < i1; ++i) {
     const long long tk = clock64();
     uint32_t item, res = 0u;
@@ -1869,7 +1949,7 @@ __device__ void regionWork(const KParams &p, BlockSmem &b, uint32_t t, uint32_t 
     }
   }
   if (r == 0) {
-    if ((p.flags & kFlagDigest) || event) digestSlice<SPW>(p, t);
+    if ((p.flags & kFlagDigest) || event) digestSlice<SPW>(p, t, block);
     if (p.flags & kFlagSlots) eventRegion0<SPW>(p, retBits, retCnt);  // the cycle's list, also when empty
   } else {
     if (event) eventRegion1(p, gtid, gthreads);
@@ -1896,11 +1976,12 @@ __global__ void __launch_bounds__(LV == kLevelsProgramResident ? kResidentThread
     __shared__ uint32_t itemLists[2 * kItemListWords];
     loadItemLists(p, b, itemLists);
   }
-  const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
+  const uint32_t block = workBlock<LV>();
+  const uint32_t gtid = block * blockDim.x + threadIdx.x, gthreads = p.nBlocks * blockDim.x;
   const uint32_t cEnd = c0 + nCycles;
   uint32_t gen = 0;
   if (p.flags & kFlagStimulus) {
-    applyStimulus<SPW>(p, c0, gtid, gthreads);
+    if (block < p.nBlocks) applyStimulus<SPW>(p, c0, gtid, gthreads);
     if (!gridSync(p, gen)) return;
   }
   const bool slots = (p.flags & kFlagSlots) != 0;
@@ -1914,11 +1995,11 @@ __global__ void __launch_bounds__(LV == kLevelsProgramResident ? kResidentThread
       const long long tStart = clock64();
       regionWork<SPW, G, LV>(p, b, t, r, event, retBits, retCnt, cEnd, c0);
       if (!gridSync(p, gen)) return;
-      if ((p.flags & kFlagProfile) && threadIdx.x == 0 && t >= c0 + 100 && t < c0 + 200) {
+      if ((p.flags & kFlagProfile) && threadIdx.x == 0 && block < p.nBlocks && t >= c0 + 100 && t < c0 + 200) {
         const long long total = clock64() - tStart;
         const uint32_t pc = t - c0 - 100;
         const uint32_t *ib = p.itemBegin + r * (p.nBlocks + 1);
-        for (uint32_t i = __ldg(ib + blockIdx.x); i < __ldg(ib + blockIdx.x + 1); ++i) {
+        for (uint32_t i = __ldg(ib + block); i < __ldg(ib + block + 1); ++i) {
           const uint32_t item = __ldg(p.items + i);
           if ((item >> 20) != 0) continue;
           const uint32_t pid = item & 0xFFFFFu;
@@ -1927,14 +2008,14 @@ __global__ void __launch_bounds__(LV == kLevelsProgramResident ? kResidentThread
       }
     }
     if ((p.flags & kFlagStopExit) && (p.flags & kFlagStimulus) && t + 1 < cEnd) {
-      applyStimulus<SPW>(p, t + 1, gtid, gthreads);
+      if (block < p.nBlocks) applyStimulus<SPW>(p, t + 1, gtid, gthreads);
       if (!gridSync(p, gen)) return;
     }
     if (event) {
       eventAdmit<SPW>(p, t, gtid, gthreads);
       if (!gridSync(p, gen)) return;
     }
-    if ((p.flags & kFlagCountCycles) && blockIdx.x == 0 && threadIdx.x == 0) *p.realCycles += 1;
+    if ((p.flags & kFlagCountCycles) && block == 0 && threadIdx.x == 0) *p.realCycles += 1;
     // every block reads the words after the cycle's last barrier: same decision
     if (scan) {
       hint = __ldcg(p.eventHint + ((t + 1u) & 1u));  // this scan's bound, lowered by the admissions
@@ -1950,7 +2031,7 @@ __global__ void __launch_bounds__(LV == kLevelsProgramResident ? kResidentThread
     uint32_t any = 0;
     for (uint32_t s = threadIdx.x; s < p.nStreams; s += blockDim.x) any |= __ldcg(p.stop + s);
     const int stopped = __syncthreads_or(int(any));
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
       p.status[1] = stopped ? 1u : 0u;
       p.status[0] = __ldcg(p.err);
     }
@@ -1987,7 +2068,8 @@ __global__ void __launch_bounds__(1024) regionKernel(const KParams p, uint32_t k
 // source; each instantiating translation unit takes one form and one source.
 template <int LV>
 void *cycleKernelPtrT(int spw, int G) {
-  if (spw == 1) return reinterpret_cast<void *>(&cycleKernel<1, 1, LV>);
+  if constexpr (LV != kLevelsProgramTeams)
+    if (spw == 1) return reinterpret_cast<void *>(&cycleKernel<1, 1, LV>);
   if (G == 8) return reinterpret_cast<void *>(&cycleKernel<8, 8, LV>);
   if (G == 4) return reinterpret_cast<void *>(&cycleKernel<8, 4, LV>);
   if (G == 2) return reinterpret_cast<void *>(&cycleKernel<8, 2, LV>);
@@ -1996,7 +2078,8 @@ void *cycleKernelPtrT(int spw, int G) {
 
 template <int LV>
 void *regionKernelPtrT(int spw, int G) {
-  if (spw == 1) return reinterpret_cast<void *>(&regionKernel<1, 1, LV>);
+  if constexpr (LV != kLevelsProgramTeams)
+    if (spw == 1) return reinterpret_cast<void *>(&regionKernel<1, 1, LV>);
   if (G == 8) return reinterpret_cast<void *>(&regionKernel<8, 8, LV>);
   if (G == 4) return reinterpret_cast<void *>(&regionKernel<8, 4, LV>);
   if (G == 2) return reinterpret_cast<void *>(&regionKernel<8, 2, LV>);

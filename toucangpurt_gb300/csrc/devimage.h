@@ -125,8 +125,15 @@ constexpr uint32_t kResidentItems = 8u;  // items of a region per block, at most
 
 // Where a block reads its exec levels: staged per level into shared memory
 // (or, level by level, from global memory), resident there for the launch,
-// warp programs, or warp programs resident there for the launch.
-enum : int { kLevelsStaged = 0, kLevelsResident = 1, kLevelsProgram = 2, kLevelsProgramResident = 3 };
+// warp programs, warp programs resident there for the launch, or warp programs
+// run by teams of warps in one block per SM.
+enum : int {
+  kLevelsStaged = 0,
+  kLevelsResident = 1,
+  kLevelsProgram = 2,
+  kLevelsProgramResident = 3,
+  kLevelsProgramTeams = 4
+};
 
 // Kernel parameters (passed by value).
 struct KParams {
@@ -238,5 +245,13 @@ enum : uint32_t {
 };
 
 constexpr uint32_t kLutTablePadded = 4656;  // 4642 rounded up to 16 bytes
+
+// Shared memory of teams (kLevelsProgramTeams): the byte table to whole rows of
+// 128 bytes, the nibble table (8 entries a row, once per lane), value pools.
+// At least as much as an index that no static check bounded can reach
+// (lutIndex 4,641 and operands 15, 15, 15).
+constexpr uint32_t kByteTableBytes = 4736, kNibbleRows = 581;
+constexpr uint32_t kTeamTableBytes = kByteTableBytes + 128u * kNibbleRows;
+constexpr uint32_t kTeamSmemMin = kByteTableBytes + 128u * 1093u;
 
 }  // namespace tgs

@@ -13,6 +13,7 @@ struct LaunchCfg {
   int spw = 1, G = 1;
   int lv = kLevelsStaged;  // where blocks read the exec levels
   uint32_t blocks = 1, threads = 256;
+  uint32_t teams = 1;        // teams of `threads` threads per block (kLevelsProgramTeams)
   size_t smem = 0;
   cudaStream_t stream = nullptr;
 };
@@ -34,6 +35,8 @@ void *regionKernelResident(int spw, int G);
 void *cycleKernelProgram(int spw, int G);
 void *cycleKernelProgramResident(int spw, int G);
 void *regionKernelProgram(int spw, int G);
+void *cycleKernelProgramTeams(int spw, int G);
+void *regionKernelProgramTeams(int spw, int G);
 // blocks that own their streams (kernels_own_streams.cu), 8 streams per word
 void *ownStreamsKernelFor(int G);
 cudaError_t launchOwnStreams(const LaunchCfg &c, const KParams &p, uint32_t c0, uint32_t n);

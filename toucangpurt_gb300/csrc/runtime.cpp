@@ -102,6 +102,9 @@ struct tgs_sim {
   uint32_t spw = 1, groups = 1, gpad = 1, nStreams = 1, regSlots = 4, exgSlots = 4, stageWords = 0;
   uint32_t progResWords = 0;  // words of a block's resident partition images (0: programs read from global memory)
   size_t progResSmem = 0;
+  // teams of warps, one block per SM (0 teams: not used); the work blocks are lc.blocks
+  uint32_t teams = 0;
+  size_t teamSmem = 0;
   // blocks that own their streams: one block per group block, its items and images
   uint32_t ownWords = 0;
   bool ownCounts = true;  // a block's cycle counter (at most the sum of the queue's lengths) fits 32 bits
@@ -465,6 +468,7 @@ void configure(tgs_sim *h) {
   h->resWords = 0;
   h->progResWords = 0;
   h->ownWords = 0;
+  h->teams = 0;
   // Where a block's partitions lie in its resident area: (source word, words)
   // of each partition, one copy per block and partition.  Returns the words of
   // the largest block.
@@ -572,6 +576,31 @@ void configure(tgs_sim *h) {
         }
       }
       TGS_CUDA(cudaStreamSynchronize(h->stream));  // the vectors end with this scope
+    }
+  }
+  // Several blocks' worth of work per SM, 8 streams per word: the blocks of an
+  // SM as teams of one block that share the byte and the nibble table (the
+  // shared-memory pipe bounds such launches; with one block per SM latency
+  // does, which the nibble lookups' longer chain adds to).
+  if (program && h->spw == 8) {
+    const uint32_t sms = uint32_t(h->props.multiProcessorCount), T = (B + sms - 1) / sms;
+    const size_t need = kTeamTableBytes + size_t(T) * vpBytes, smemT = std::max(need, size_t(kTeamSmemMin));
+    if (T >= 2 && T <= 15 && T * h->lc.threads <= 1024 && smemT <= size_t(h->props.sharedMemPerBlockOptin)) {
+      bool fits = true;
+      for (void *k : {cycleKernelFor(8, G, kLevelsProgramTeams), regionKernelFor(8, G, kLevelsProgramTeams)}) {
+        cudaFuncAttributes ta{};
+        TGS_CUDA(cudaFuncGetAttributes(&ta, k));
+        fits = fits && smemT + ta.sharedSizeBytes <= size_t(h->props.sharedMemPerBlockOptin);
+        if (!fits) break;
+        TGS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemT)));
+        int n = 0;
+        TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, int(T * h->lc.threads), smemT));
+        fits = n > 0;
+      }
+      if (fits) {
+        h->teams = T;
+        h->teamSmem = smemT;
+      }
     }
   }
   if (!program) {
@@ -766,22 +795,37 @@ void requireLoaded(tgs_sim *h, bool ordered = false) {
   }
 }
 
+// The launch of a run with these flags: teams where they are set up; queued
+// streams (whose retirements every block looks for) and micro-partition
+// profiles take the block form.
+LaunchCfg launchCfg(const tgs_sim *h, uint32_t flags) {
+  LaunchCfg c = h->lc;
+  if (h->teams && !(flags & (kFlagSlots | kFlagProfileMP))) {
+    c.lv = kLevelsProgramTeams;
+    c.blocks = uint32_t(h->props.multiProcessorCount);
+    c.teams = h->teams;
+    c.smem = h->teamSmem;
+  }
+  return c;
+}
+
 // Graph form: chunks of up to 32 cycles (two region launches and an admit
 // launch per cycle) captured once and replayed.  The kernels read the cycle,
 // the event cursor and the end cycle from device words, so a chunk captured
 // for one call serves every later call with the same launch parameters.
 cudaGraphExec_t graphChunk(tgs_sim *h, const KParams &p, uint32_t k, bool admit) {
-  std::vector<uint8_t> key(sizeof(KParams) + 7 * sizeof(uint32_t));
+  const LaunchCfg c = launchCfg(h, p.flags);
+  std::vector<uint8_t> key(sizeof(KParams) + 9 * sizeof(uint32_t));
   std::memcpy(key.data(), &p, sizeof(KParams));
-  const uint32_t tail[7] = {k, admit ? 1u : 0u, uint32_t(h->lc.spw), uint32_t(h->lc.G), h->lc.blocks, h->lc.threads,
-                            uint32_t(h->lc.smem)};
+  const uint32_t tail[9] = {k,         admit ? 1u : 0u,    uint32_t(c.spw), uint32_t(c.G), c.blocks,
+                            c.threads, uint32_t(c.smem), uint32_t(c.lv),  c.teams};
   std::memcpy(key.data() + sizeof(KParams), tail, sizeof(tail));
   for (auto &g : h->graphs)
     if (g.key == key) return g.exec;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   TGS_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  const cudaError_t e = enqueueGraphChunk(h->lc, p, k, admit);
+  const cudaError_t e = enqueueGraphChunk(c, p, k, admit);
   const cudaError_t e2 = cudaStreamEndCapture(h->stream, &graph);
   if (e != cudaSuccess || e2 != cudaSuccess) {
     if (graph) cudaGraphDestroy(graph);
@@ -863,7 +907,7 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     p.resSrc = h->partImages.p;
     TGS_CUDA(launchCycles(c, p, c0, n));
   } else {
-    TGS_CUDA(launchCycles(h->lc, h->kp, c0, n));
+    TGS_CUDA(launchCycles(launchCfg(h, flags), h->kp, c0, n));
   }
   h->lastLaunches = 1;
 }
