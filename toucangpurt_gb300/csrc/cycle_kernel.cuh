@@ -318,6 +318,21 @@ __device__ __forceinline__ void copyInG(uint32_t dst, const uint32_t *__restrict
   }
 }
 
+// global (mutable state, L1 bypass) -> registers
+template <int G>
+__device__ __forceinline__ void readStateG(const uint32_t *__restrict__ src, uint32_t (&v)[G]) {
+  if constexpr (G == 4) {
+    const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(src));
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else if constexpr (G == 2) {
+    const uint2 q = __ldcg(reinterpret_cast<const uint2 *>(src));
+    v[0] = q.x; v[1] = q.y;
+  } else {
+    v[0] = __ldcg(src);
+  }
+}
+constexpr uint32_t kL0Ahead = 2;
+
 // value pool -> global
 template <int G>
 __device__ __forceinline__ void copyOutG(uint32_t *__restrict__ dst, uint32_t src) {
@@ -1172,11 +1187,27 @@ __device__ void evalItem(const KParams &p, uint32_t item, uint32_t vp, uint32_t 
   {
     const uint32_t n = d.l0Count;
     const uint32_t *pool = d.l0Exchange ? p.exg : p.regs;
-    for (uint32_t i = tid; i < n; i += nthr) {
-      const uint32_t s = word(d.l0Off + i);
-      const uint32_t r = (word(d.l0Off + n + (i >> 1)) >> ((i & 1u) * 16)) & 0xFFFFu;
-      copyInG<G>(vpAddr<G>(vp, r, 0), pool + size_t(s) * p.gpad + gb * G);
+    auto from = [&](uint32_t i) { return pool + size_t(word(d.l0Off + i)) * p.gpad + gb * G; };
+    auto to = [&](uint32_t i) {
+      return vpAddr<G>(vp, (word(d.l0Off + n + (i >> 1)) >> ((i & 1u) * 16)) & 0xFFFFu, 0);
+    };
+    uint32_t i = tid;
+    if constexpr (PRES && G <= 4) {
+      // kL0Ahead reads of a thread in flight (few blocks, registers to spare): a
+      // partition with a few more reads than threads waited for the L2 twice
+      // (4K-LUT design, one stream, 1,000 cycles 5.62 -> 5.46 ms, queued streams
+      // 20.1 -> 19.5; 3 and 4 reads 5.49 and 5.62)
+      for (; i < n; i += kL0Ahead * nthr) {
+        uint32_t v[kL0Ahead][G];
+#pragma unroll
+        for (uint32_t u = 0; u < kL0Ahead; ++u)
+          if (i + u * nthr < n) readStateG<G>(from(i + u * nthr), v[u]);
+#pragma unroll
+        for (uint32_t u = 0; u < kL0Ahead; ++u)
+          if (i + u * nthr < n) storeG<G>(to(i + u * nthr), v[u]);
+      }
     }
+    for (; i < n; i += nthr) copyInG<G>(to(i), from(i));
   }
   if (cap) stageCopyWait();  // the first level's pieces, before the barrier that publishes them
   teamSync<LV>();
