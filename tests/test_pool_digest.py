@@ -21,8 +21,8 @@ def _digests(pools):
 # tails of 0..15 bytes; 4 MiB and more, where the bits above 2^30 of the mixed
 # index change inside a 16-byte vector; 1, 7, 8, 9 and 17 pools
 @pytest.mark.parametrize("size", [1, 15, 16, 17, 4099, (1 << 22) + 5])
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 17])
-@pytest.mark.parametrize("fill", ["equal", "nibbles", "bytes"])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 17, 130])
+@pytest.mark.parametrize("fill", ["equal", "sparse", "nibbles", "bytes"])
 @pytest.mark.parametrize("offset", [0, 3])
 def test_pool_digests(built, size, n, fill, offset):
     torch = pytest.importorskip("torch")
@@ -30,6 +30,12 @@ def test_pool_digests(built, size, n, fill, offset):
         pytest.skip("the long pool with two pool counts only")
     rng = np.random.default_rng(size + n)
     host = rng.integers(0, 256 if fill == "bytes" else 16, (n, size)).astype(np.uint8)
+    if fill == "sparse":  # equal but for a few bytes of every pool, several in one 16-byte piece among them
+        host[:] = host[0]
+        for k in range(n):
+            at = rng.integers(0, size, max(1, size // 40))
+            host[k, at] = rng.integers(0, 256, at.size)
+            host[k, size // 3:size // 3 + 5] ^= k
     if fill == "equal":
         host[:] = host[0]
         host[n // 2, size // 2] ^= 1

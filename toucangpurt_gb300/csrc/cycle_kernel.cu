@@ -77,16 +77,18 @@ __global__ void __launch_bounds__(256) initMemsKernel(const uint8_t *__restrict_
 // each of them.  Streams' memories start equal and are written sparsely, so a
 // thread computes the 16 terms of the first stream once and, for every other
 // stream, only what differs from it: nothing when the warp's 512 bytes are
-// equal, the differing bytes' terms when up to half of the lanes differ, all
-// 16 terms (17 instructions a byte beside the index part) otherwise.  A warp's
-// correction is summed with three 27-bit reductions into its own row of sums.
-// Measured, 64 pools of 128 MiB (start: 17.5 ms in every case, bound by 27
-// instructions of whole mixes per byte and one-byte loads): equal 1.19 ms
-// (7.2 TB/s, bound by HBM), 0.5 % of a pool's bytes differing 4.3 ms, all
-// random 12.7 ms (both bound by instructions).  Half the lanes as the line:
-// 8 lanes 8.2 ms, 16 and 24 lanes 4.8 ms at 0.5 %.  64 registers (4 blocks an
-// SM) over 80 and 128 (index parts kept): 4.3 / 4.8 / 5.4 ms at 0.5 %.
+// equal; the differing bytes when up to half of the lanes differ, gathered by
+// the warp and taken 32 at a time, one a lane; all 16 terms (17 instructions a
+// byte beside the index part) otherwise.
+// Measured, 64 pools of 128 MiB (17.5 ms in every case when each byte took the
+// whole 27-instruction mix and a thread read one byte a step): equal 1.25 ms
+// (6.9 TB/s, bound by HBM), 0.5 % of a pool's bytes differing 3.25 ms (4.3 with
+// each lane taking its own bytes, a few of 32 lanes at work), all random
+// 12.9 ms, both bound by instructions.  Half the lanes as the line: with 8
+// lanes 8.2 ms at 0.5 %, 16 and 24 lanes 4.8 ms.  64 registers (4 blocks an SM)
+// over 80 and 128 (index parts kept): 4.3 / 4.8 / 5.4 ms at 0.5 %.
 constexpr uint32_t kDigestThreads = 256, kDigestStreams = 64;
+constexpr uint32_t kDigestQueue = 64;   // differing bytes a warp gathers
 constexpr uint32_t kDigestSparse = 16;  // lanes of a warp that differ, up to which their bytes are taken one by one
 
 __global__ void __launch_bounds__(kDigestThreads, 4)
@@ -94,13 +96,15 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
                     unsigned long long *__restrict__ out) {
   __shared__ unsigned long long sum[kDigestThreads / 32][kDigestStreams];  // per warp: stream's sum less the first stream's (wrapping)
   __shared__ unsigned long long sum0;
+  __shared__ uint32_t piece[kDigestThreads / 32u][kDigestStreams][3], queue[kDigestThreads / 32u][kDigestQueue];
   const uint32_t s0 = blockIdx.y * kDigestStreams, ns = min(kDigestStreams, nStreams - s0);
   const uint8_t *base = mems + s0 * stride;
   for (uint32_t i = threadIdx.x; i < kDigestThreads / 32u * kDigestStreams; i += kDigestThreads) (&sum[0][0])[i] = 0;
+  for (uint32_t i = threadIdx.x; i < kDigestThreads / 32u * kDigestStreams * 3u; i += kDigestThreads) (&piece[0][0][0])[i] = 0;
   if (threadIdx.x == 0) sum0 = 0;
   __syncthreads();
   unsigned long long acc0 = 0;
-  const uint32_t vecs = size / 16u, lane = threadIdx.x & 31u;
+  const uint32_t vecs = size / 16u, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   // whole warps iterate together (a lane past the end repeats the last vector with weight 0)
   for (uint32_t w = blockIdx.x * kDigestThreads + threadIdx.x - lane; w < vecs; w += gridDim.x * kDigestThreads) {
     const bool in = w + lane < vecs;
@@ -130,37 +134,71 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
     };
     const unsigned long long first = sum16(f);
     if (in) acc0 += first;
+    uint32_t queued = 0;  // the same in every lane
+    // the terms of up to 32 queued bytes, one a lane: added to their streams'
+    // pieces (22, 21 and 21 bits: an iteration adds at most 512 times to one)
+    auto flush = [&]() {
+      __syncwarp();
+      if (lane < queued) {
+        const uint32_t e = queue[warp][lane], a = e & 0xFFu, b = (e >> 8) & 0xFFu, k = e >> 25;
+        const unsigned long long i = 16ull * w + ((e >> 16) & 511u);
+        unsigned long long s;
+        if ((a | b) < 0x80u) {
+          const MixIndex mix(i);
+          s = mix(a) - mix(b);
+        } else {
+          s = dmix64(i << 8 | a) - dmix64(i << 8 | b);
+        }
+        atomicAdd(&piece[warp][k][0], uint32_t(s) & 0x3FFFFFu);
+        atomicAdd(&piece[warp][k][1], uint32_t(s >> 22) & 0x1FFFFFu);
+        atomicAdd(&piece[warp][k][2], uint32_t(s >> 43));
+      }
+      __syncwarp();
+    };
+    bool any = false;
     auto other = [&](uint32_t k, const uint4 &q) {
       const uint4 d = make_uint4(q.x ^ f.x, q.y ^ f.y, q.z ^ f.z, q.w ^ f.w);
       const bool differs = in && (d.x | d.y | d.z | d.w) != 0u;
       const uint32_t lanes = __ballot_sync(kFull, differs);
       if (lanes == 0u) return;
-      unsigned long long s = 0;
-      if (__popc(lanes) <= kDigestSparse) {
-        if (differs) {
-          // one bit per differing byte
-          auto bytes = [](uint32_t x) { return ((__vcmpne4(x, 0u) & 0x08040201u) * 0x01010101u) >> 24; };
-          for (uint32_t r = bytes(d.x) | bytes(d.y) << 4 | bytes(d.z) << 8 | bytes(d.w) << 12; r; r &= r - 1u) {
-            const uint32_t j = uint32_t(__ffs(int(r))) - 1u, sh = 8u * (j & 3u);
-            const uint32_t a = ((j < 8 ? (j < 4 ? q.x : q.y) : (j < 12 ? q.z : q.w)) >> sh) & 0xFFu;
-            const uint32_t b = ((j < 8 ? (j < 4 ? f.x : f.y) : (j < 12 ? f.z : f.w)) >> sh) & 0xFFu;
-            if ((a | b) < 0x80u) {
-              const MixIndex mix(i0 + j);
-              s += mix(a) - mix(b);
-            } else {
-              s += dmix64((i0 + j) << 8 | a) - dmix64((i0 + j) << 8 | b);
-            }
-          }
-        }
-      } else if (in) {
-        s = sum16(q) - first;
+      if (__popc(lanes) > kDigestSparse) {
+        // sum over the warp in three pieces that fit 32 bits
+        const unsigned long long s = in ? sum16(q) - first : 0ull;
+        const uint32_t x0 = __reduce_add_sync(kFull, uint32_t(s) & 0x7FFFFFFu);
+        const uint32_t x1 = __reduce_add_sync(kFull, uint32_t(s >> 27) & 0x7FFFFFFu);
+        const uint32_t x2 = __reduce_add_sync(kFull, uint32_t(s >> 54));
+        if (lane == 0)
+          sum[warp][k] += (unsigned long long)x0 + ((unsigned long long)x1 << 27) + ((unsigned long long)x2 << 54);
+        return;
       }
-      // sum over the warp in three pieces that fit 32 bits
-      const uint32_t s0 = __reduce_add_sync(kFull, uint32_t(s) & 0x7FFFFFFu);
-      const uint32_t s1 = __reduce_add_sync(kFull, uint32_t(s >> 27) & 0x7FFFFFFu);
-      const uint32_t s2 = __reduce_add_sync(kFull, uint32_t(s >> 54));
-      if (lane == 0)
-        sum[threadIdx.x / 32u][k] += (unsigned long long)s0 + ((unsigned long long)s1 << 27) + ((unsigned long long)s2 << 54);
+      any = true;
+      // one bit per differing byte, then a byte of each lane a round
+      auto bytes = [](uint32_t x) {
+        return (((((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) >> 7 & 0x01010101u) * 0x01020408u >> 24) & 15u;
+      };
+      uint32_t m = 0;
+      if (differs) m = bytes(d.x) | bytes(d.y) << 4 | bytes(d.z) << 8 | bytes(d.w) << 12;
+      for (uint32_t left = lanes; left; left = __ballot_sync(kFull, m != 0u)) {
+        const uint32_t n = uint32_t(__popc(left));
+        if (queued + n > kDigestQueue) {
+          // full: the first 32 are taken, the rest moves down
+          const uint32_t rest = queued - 32u;
+          const uint32_t keep = queued;
+          queued = 32u;
+          flush();
+          if (lane < rest) queue[warp][lane] = queue[warp][32u + lane];
+          queued = keep - 32u;
+          __syncwarp();
+        }
+        if (m) {
+          const uint32_t j = uint32_t(__ffs(int(m))) - 1u, sh = 8u * (j & 3u);
+          m &= m - 1u;
+          const uint32_t a = ((j < 8 ? (j < 4 ? q.x : q.y) : (j < 12 ? q.z : q.w)) >> sh) & 0xFFu;
+          const uint32_t b = ((j < 8 ? (j < 4 ? f.x : f.y) : (j < 12 ? f.z : f.w)) >> sh) & 0xFFu;
+          queue[warp][queued + uint32_t(__popc(left & ((1u << lane) - 1u)))] = a | b << 8 | (16u * lane + j) << 16 | k << 25;
+        }
+        queued += n;
+      }
     };
     const uint8_t *at = reinterpret_cast<const uint8_t *>(src) + stride;
     uint32_t k = 1;
@@ -172,6 +210,23 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
       for (int u = 0; u < 8; ++u) other(k + u, q[u]);
     }
     for (; k < ns; ++k, at += stride) other(k, __ldg(reinterpret_cast<const uint4 *>(at)));
+    if (any) {
+      // what is still queued, then the pieces
+      if (queued > 32u) {
+        const uint32_t rest = queued - 32u;
+        queued = 32u;
+        flush();
+        if (lane < rest) queue[warp][lane] = queue[warp][32u + lane];
+        queued = rest;
+      }
+      flush();
+      for (uint32_t s = lane; s < ns; s += 32u) {
+        sum[warp][s] += (unsigned long long)piece[warp][s][0] + ((unsigned long long)piece[warp][s][1] << 22) +
+                        ((unsigned long long)piece[warp][s][2] << 43);
+        piece[warp][s][0] = piece[warp][s][1] = piece[warp][s][2] = 0u;
+      }
+      __syncwarp();
+    }
   }
   __syncthreads();
   // the last size % 16 bytes
