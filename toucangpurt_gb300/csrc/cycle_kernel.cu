@@ -75,8 +75,8 @@ __global__ void __launch_bounds__(256) initMemsKernel(const uint8_t *__restrict_
 // Digest of one pool per stream: sum over i of mix64(i << 8 | v_i).
 // A block takes up to kDigestStreams streams, a thread the same 16 bytes of
 // each of them.  Streams' memories start equal and are written sparsely, so a
-// thread computes the 16 terms of the first stream once and, for every other
-// stream, only what differs from it: nothing when the warp's 512 bytes are
+// thread computes the 16 terms of the initial image (of the first stream,
+// where there is none) once and, for every stream, only what differs from it: nothing when the warp's 512 bytes are
 // equal; the differing bytes when up to half of the lanes differ, gathered by
 // the warp and taken 32 at a time, one a lane; all 16 terms (17 instructions a
 // byte beside the index part) otherwise.
@@ -93,12 +93,16 @@ constexpr uint32_t kDigestSparse = 16;  // lanes of a warp that differ, up to wh
 
 __global__ void __launch_bounds__(kDigestThreads, 4)
     memDigestKernel(const uint8_t *__restrict__ mems, unsigned long long stride, uint32_t size, uint32_t nStreams,
-                    unsigned long long *__restrict__ out) {
+                    const uint8_t *__restrict__ image, unsigned long long *__restrict__ out) {
   __shared__ unsigned long long sum[kDigestThreads / 32][kDigestStreams];  // per warp: stream's sum less the first stream's (wrapping)
   __shared__ unsigned long long sum0;
   __shared__ uint32_t piece[kDigestThreads / 32u][kDigestStreams][3], queue[kDigestThreads / 32u][kDigestQueue];
   const uint32_t s0 = blockIdx.y * kDigestStreams, ns = min(kDigestStreams, nStreams - s0);
   const uint8_t *base = mems + s0 * stride;
+  // what the streams are compared with: the initial image (a byte the first
+  // stream wrote would differ from every other), or the first stream
+  const uint8_t *ref = image ? image : base;
+  const uint32_t kFirst = image ? 0u : 1u;
   for (uint32_t i = threadIdx.x; i < kDigestThreads / 32u * kDigestStreams; i += kDigestThreads) (&sum[0][0])[i] = 0;
   for (uint32_t i = threadIdx.x; i < kDigestThreads / 32u * kDigestStreams * 3u; i += kDigestThreads) (&piece[0][0][0])[i] = 0;
   if (threadIdx.x == 0) sum0 = 0;
@@ -110,7 +114,7 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
     const bool in = w + lane < vecs;
     const uint32_t v = in ? w + lane : vecs - 1u;
     const uint4 *src = reinterpret_cast<const uint4 *>(base) + v;
-    const uint4 f = __ldg(src);
+    const uint4 f = __ldg(reinterpret_cast<const uint4 *>(ref) + v);
     // the 16 indices share z >> 30 (and so its low byte) unless their low 30
     // bits wrap; values of 0x80 and above, which a pool may hold when the
     // caller wrote them, may carry out of the low byte: both take the full mix
@@ -200,8 +204,8 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
         queued += n;
       }
     };
-    const uint8_t *at = reinterpret_cast<const uint8_t *>(src) + stride;
-    uint32_t k = 1;
+    const uint8_t *at = reinterpret_cast<const uint8_t *>(src) + kFirst * stride;
+    uint32_t k = kFirst;
     for (; k + 8 <= ns; k += 8, at += 8 * stride) {
       uint4 q[8];
 #pragma unroll
@@ -232,9 +236,9 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
   // the last size % 16 bytes
   if (blockIdx.x == 0 && threadIdx.x < size % 16u) {
     const uint32_t i = size - size % 16u + threadIdx.x;
-    const unsigned long long t0 = dmix64((unsigned long long)i << 8 | base[i]);
+    const unsigned long long t0 = dmix64((unsigned long long)i << 8 | ref[i]);
     acc0 += t0;
-    for (uint32_t k = 1; k < ns; ++k)
+    for (uint32_t k = kFirst; k < ns; ++k)
       atomicAdd(&sum[0][k], dmix64((unsigned long long)i << 8 | base[k * stride + i]) - t0);
   }
   for (int o = 16; o > 0; o >>= 1) acc0 += __shfl_xor_sync(kFull, acc0, o);
@@ -432,7 +436,7 @@ cudaError_t launchRegDigestOne(const uint32_t *regs, uint32_t slots, uint32_t gp
 }
 
 cudaError_t launchMemDigest(const uint8_t *mems, unsigned long long stride, uint32_t size, uint32_t nStreams,
-                            unsigned long long *out, cudaStream_t st) {
+                            const uint8_t *image, unsigned long long *out, cudaStream_t st) {
   if (size == 0 || nStreams == 0) return cudaSuccess;
   if (((reinterpret_cast<uintptr_t>(mems) | (nStreams > 1 ? stride : 0ull)) & 15u) != 0u) {
     dim3 grid(std::max<uint32_t>(1, std::min<uint32_t>(1024, (size + 255) / 256)), nStreams);
@@ -443,7 +447,7 @@ cudaError_t launchMemDigest(const uint8_t *mems, unsigned long long stride, uint
   const uint32_t gy = (nStreams + kDigestStreams - 1) / kDigestStreams;
   const uint32_t full = (size / 16u + kDigestThreads - 1) / kDigestThreads;
   dim3 grid(std::max<uint32_t>(1, std::min<uint32_t>(full, std::max<uint32_t>(1, 1216u / gy))), gy);
-  memDigestKernel<<<grid, kDigestThreads, 0, st>>>(mems, stride, size, nStreams, out);
+  memDigestKernel<<<grid, kDigestThreads, 0, st>>>(mems, stride, size, nStreams, nStreams >= 8u ? image : nullptr, out);
   return cudaGetLastError();
 }
 

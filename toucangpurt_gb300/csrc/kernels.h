@@ -49,8 +49,9 @@ cudaError_t launchRegDigest(int spw, const uint32_t *regs, uint32_t slots, uint3
                             unsigned long long *out, cudaStream_t st);
 cudaError_t launchRegDigestOne(const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t g, uint32_t k,
                                unsigned long long *out, cudaStream_t st);
+// image: the pools' initial contents (16-byte aligned, whole 16-byte pieces), or null
 cudaError_t launchMemDigest(const uint8_t *mems, unsigned long long stride, uint32_t size, uint32_t nStreams,
-                            unsigned long long *out, cudaStream_t st);
+                            const uint8_t *image, unsigned long long *out, cudaStream_t st);
 cudaError_t launchGatherRegs(const uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t g, uint32_t k, uint8_t *out,
                              cudaStream_t st);
 cudaError_t launchScatterRegs(uint32_t *regs, uint32_t slots, uint32_t gpad, uint32_t g, uint32_t k, const uint8_t *in,

@@ -50,7 +50,7 @@ extern "C" int tgs_pool_digests_noalloc(const uint8_t *pools, uint64_t stride, u
     unsigned long long *acc = scratchForCurrentDevice();
     // the array keeps the previous call's sums: clear the part this call uses
     cudaError_t e = cudaMemsetAsync(acc, 0, size_t(n_pools) * sizeof(unsigned long long), nullptr);
-    if (e == cudaSuccess) e = launchMemDigest(pools, stride, uint32_t(bytes), n_pools, acc, nullptr);
+    if (e == cudaSuccess) e = launchMemDigest(pools, stride, uint32_t(bytes), n_pools, nullptr, acc, nullptr);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(digests, acc, size_t(n_pools) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);

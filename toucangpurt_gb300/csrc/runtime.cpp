@@ -1705,7 +1705,7 @@ int tgs_state_digest(tgs_sim *h, uint32_t s, uint64_t *rd, uint64_t *md) {
     TGS_CUDA(cudaMemsetAsync(h->outA.p + s, 0, 8, h->stream));
     TGS_CUDA(cudaMemsetAsync(h->outB.p + s, 0, 8, h->stream));
     TGS_CUDA(launchRegDigestOne(h->regs.p, h->design.regPoolSize, h->gpad, g, k, h->outA.p + s, h->stream));
-    TGS_CUDA(launchMemDigest(h->mems.p + size_t(s) * h->memStride, h->memStride, h->design.memPoolSize, 1,
+    TGS_CUDA(launchMemDigest(h->mems.p + size_t(s) * h->memStride, h->memStride, h->design.memPoolSize, 1, nullptr,
                              h->outB.p + s, h->stream));
     unsigned long long a = 0, b = 0;
     TGS_CUDA(cudaMemcpyAsync(&a, h->outA.p + s, 8, cudaMemcpyDeviceToHost, h->stream));
@@ -2079,7 +2079,7 @@ void batchRun(tgs_sim *h, const tgs_batch *job, tgs_batch_result *res) {
       TGS_CUDA(cudaMemcpyAsync(res->final_reg_digest, h->outA.p, n * 8ull, cudaMemcpyDeviceToHost, s));
     }
     if (res->final_mem_digest) {
-      TGS_CUDA(launchMemDigest(h->mems.p, h->memStride, h->design.memPoolSize, n, h->outB.p, s));
+      TGS_CUDA(launchMemDigest(h->mems.p, h->memStride, h->design.memPoolSize, n, h->initMems.p, h->outB.p, s));
       TGS_CUDA(cudaMemcpyAsync(res->final_mem_digest, h->outB.p, n * 8ull, cudaMemcpyDeviceToHost, s));
     }
   }
