@@ -1530,15 +1530,22 @@ __device__ __forceinline__ uint32_t sumStreams(unsigned long long (&acc)[SPW], u
 // A warp takes a chunk of registers of one group; the index part of the mix is
 // computed once for the 8 streams of a word (17 instead of 27 instructions a
 // value).  Chunks of 256 registers, fewer (down to one per lane) while that
-// puts more warps of the grid to work and at most 128 sums meet on a stream's
-// accumulator.  The streams' states are read by one lane each (read one after
-// another, they were 6 us of the 33 us cycle of 280 queued streams).
+// puts more warps of the grid to work and few sums meet on a stream's
+// accumulator: 256 of them if the chunks were 256 registers (eight reads of a
+// lane, one after another, cost more than 128 further sums: batches of 16, 32
+// and 64 streams of a 2^20-LUT design take 5.32, 3.35 and 4.81 ms with 128
+// registers a chunk, 5.62, 3.51 and 5.00 with 256), 128 if they were smaller
+// already (64 to 32 registers with 256 sums: up to 1.4 % slower).  Up to 512
+// sums of a larger design win 5 % in one (2^21 LUTs, 16 streams) and lose
+// 0.7 % in another (1.5 million LUTs, 32 streams): left at 256 registers.
+// The streams' states are read by one lane each (read one after another, they
+// were 6 us of the 33 us cycle of 280 queued streams).
 template <int SPW>
 __device__ void digestSlice(const KParams &p, uint32_t cycle, uint32_t block) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
   const uint32_t warps = p.nBlocks * NW;
   uint32_t chunk = 256, chunks = (p.regSlots + 255u) / 256u;
-  while (chunk > 32u && chunks <= 64u && chunks * p.gpad < warps) {
+  while (chunk > 32u && chunks <= (chunk > 128u ? 128u : 64u) && chunks * p.gpad < warps) {
     chunk >>= 1;
     chunks = (p.regSlots + chunk - 1u) / chunk;
   }
