@@ -174,6 +174,10 @@ __global__ void __launch_bounds__(128, 2) mlpGradKernel(const float *__restrict_
       sm[tX + (4 * q + 3) * kRow + s] = v.w;
     }
     __syncthreads();
+    // samples from the thread's first one up to the end (the last tile's
+    // others keep zero activations: a bias may make theirs infinite where no
+    // sample's is, and 0 * infinity would reach the sums)
+    const int left = int(min(n - s0, kTile)) - int(8 * ty);
     // layer 1
     float h[4][8];
 #pragma unroll
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(128, 2) mlpGradKernel(const float *__restrict_
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) h[u][i] = fmaxf(h[u][i], 0.f);
+      for (int i = 0; i < 8; ++i) h[u][i] = i < left ? fmaxf(h[u][i], 0.f) : 0.f;
       st4(sm + tH + (4 * tx + u) * kRow + 8 * ty, h[u][0], h[u][1], h[u][2], h[u][3]);
       st4(sm + tH + (4 * tx + u) * kRow + 8 * ty + 4, h[u][4], h[u][5], h[u][6], h[u][7]);
     }
@@ -204,13 +208,13 @@ __global__ void __launch_bounds__(128, 2) mlpGradKernel(const float *__restrict_
       float o = 0.f;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        h2[u][i] = fmaxf(h2[u][i], 0.f);
+        h2[u][i] = i < left ? fmaxf(h2[u][i], 0.f) : 0.f;
         o += w3[u] * h2[u][i];
       }
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) o += __shfl_xor_sync(kFull, o, off);
       const uint32_t s = s0 + 8 * ty + i;
-      const float d = s < n ? o + b3 - y[idx ? idx[s] : s] : 0.f;
+      const float d = i < left ? o + b3 - y[idx ? idx[s] : s] : 0.f;
       dy[i] = 2.f * d * scale;
       if (tx == 0) {
         lossAcc += d * d;
