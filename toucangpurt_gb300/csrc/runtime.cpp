@@ -305,6 +305,18 @@ bool chainHeavy(const DeviceImage &img) {
   return 4 * deep > ops;
 }
 
+// The most dynamic shared memory a launch of the kernel can ask for; launches
+// up to that size are allowed from then on.  The limit belongs to the kernel,
+// not to a handle: set to one handle's size, it kept the larger launches of
+// another from starting.
+size_t mostSharedMemory(const tgs_sim *h, void *fn) {
+  cudaFuncAttributes a{};
+  TGS_CUDA(cudaFuncGetAttributes(&a, fn));
+  const size_t most = size_t(h->props.sharedMemPerBlockOptin) - a.sharedSizeBytes;
+  TGS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)));
+  return most;
+}
+
 void configure(tgs_sim *h) {
   const tgs_options &o = h->opt;
   // warp programs by default; the other forms on request, and for pools whose
@@ -378,15 +390,10 @@ void configure(tgs_sim *h) {
   }
   // the kernels' static shared memory (barrier words, retirement bitmask)
   // comes out of the same per-block limit
-  cudaFuncAttributes fa{}, fr{};
-  TGS_CUDA(cudaFuncGetAttributes(&fa, fn));
-  TGS_CUDA(cudaFuncGetAttributes(&fr, fnRegion));
-  const size_t optin = size_t(h->props.sharedMemPerBlockOptin) - std::max(fa.sharedSizeBytes, fr.sharedSizeBytes);
+  const size_t optin = std::min(mostSharedMemory(h, fn), mostSharedMemory(h, fnRegion));
   auto shape = [&](uint32_t stage) {
     h->lc.smem = kLutTablePadded + 2 * size_t(stage) * 4 + vpBytes;
     if (h->lc.smem > optin) return 0;
-    TGS_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(h->lc.smem)));
-    TGS_CUDA(cudaFuncSetAttribute(fnRegion, cudaFuncAttributeMaxDynamicSharedMemorySize, int(h->lc.smem)));
     int perSM = 0;
     TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fn, int(h->lc.threads), h->lc.smem));
     if (o.blocks_per_sm) perSM = std::min<int>(perSM, int(o.blocks_per_sm));
@@ -433,7 +440,7 @@ void configure(tgs_sim *h) {
     stage = 0;
     perSM = shape(0);
   }
-  perSM = shape(stage);  // leaves the kernel attribute at the chosen size
+  perSM = shape(stage);  // leaves lc.smem at the chosen size
   if (perSM <= 0) throw Error(TGS_ERR_RESOURCES, "no block of the cycle kernel fits on an SM with this configuration");
   // More items than blocks in flight: 4-warp blocks when they put at least
   // a quarter more items in flight (blocks on the GPU at once, up to the
@@ -507,13 +514,7 @@ void configure(tgs_sim *h) {
     const size_t smemRes = kLutTablePadded + vpBytes + size_t(words) * 4;
     void *fnRes = cycleKernelFor(int(h->spw), G, lv);
     void *fnRegionRes = regionToo ? regionKernelFor(int(h->spw), G, lv) : nullptr;
-    cudaFuncAttributes ra{}, rr{};
-    TGS_CUDA(cudaFuncGetAttributes(&ra, fnRes));
-    if (fnRegionRes) TGS_CUDA(cudaFuncGetAttributes(&rr, fnRegionRes));
-    const size_t optinRes = size_t(h->props.sharedMemPerBlockOptin) - std::max(ra.sharedSizeBytes, rr.sharedSizeBytes);
-    if (smemRes > optinRes) return 0;
-    TGS_CUDA(cudaFuncSetAttribute(fnRes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemRes)));
-    if (fnRegionRes) TGS_CUDA(cudaFuncSetAttribute(fnRegionRes, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemRes)));
+    if (smemRes > mostSharedMemory(h, fnRes) || (fnRegionRes && smemRes > mostSharedMemory(h, fnRegionRes))) return 0;
     int perSMRes = 0;
     TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMRes, fnRes, int(h->lc.threads), smemRes));
     if (o.blocks_per_sm) perSMRes = std::min<int>(perSMRes, int(o.blocks_per_sm));
@@ -550,12 +551,9 @@ void configure(tgs_sim *h) {
       if (h->spw == 8 && nGB > 1 && rp.size() == 2 && rp[0].size() == 1 && rp[1].size() == 1) {
         const uint32_t p0 = rp[0][0], p1 = rp[1][0], w0 = h->sched.imageWords[p0], w1 = h->sched.imageWords[p1];
         void *fnOwn = ownStreamsKernelFor(G);
-        cudaFuncAttributes oa{};
-        TGS_CUDA(cudaFuncGetAttributes(&oa, fnOwn));
         const uint32_t ownWords = w0 + w1 + 64u * kProgAhead;
         const size_t ownSmem = kLutTablePadded + vpBytes + size_t(ownWords) * 4;
-        if (ownSmem + oa.sharedSizeBytes <= size_t(h->props.sharedMemPerBlockOptin)) {
-          TGS_CUDA(cudaFuncSetAttribute(fnOwn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ownSmem)));
+        if (ownSmem <= mostSharedMemory(h, fnOwn)) {
           std::vector<uint32_t> items, ib(2 * (nGB + 1)), res, copy, cb(2 * (nGB + 1));
           for (uint32_t r = 0; r < 2; ++r)
             for (uint32_t b = 0; b <= nGB; ++b) {
@@ -588,11 +586,8 @@ void configure(tgs_sim *h) {
     if (T >= 2 && T <= 15 && T * h->lc.threads <= 1024 && smemT <= size_t(h->props.sharedMemPerBlockOptin)) {
       bool fits = true;
       for (void *k : {cycleKernelFor(8, G, kLevelsProgramTeams), regionKernelFor(8, G, kLevelsProgramTeams)}) {
-        cudaFuncAttributes ta{};
-        TGS_CUDA(cudaFuncGetAttributes(&ta, k));
-        fits = fits && smemT + ta.sharedSizeBytes <= size_t(h->props.sharedMemPerBlockOptin);
+        fits = fits && smemT <= mostSharedMemory(h, k);
         if (!fits) break;
-        TGS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smemT)));
         int n = 0;
         TGS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, int(T * h->lc.threads), smemT));
         fits = n > 0;
