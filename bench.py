@@ -324,8 +324,9 @@ def levels_option(a) -> int:
     return 2 if a.no_stage else {"auto": 0, "resident": 1, "global": 2, "staged": 3}[a.levels]
 
 
-def exec_levels(st) -> str:
-    return "warp programs" if st.get("program_words") else "resident" if st.get("resident_words") else "staged" if st.get("stage_words") else "global"
+def threads_per_block(st) -> int:
+    """Threads of a launched block: those of every block of work in it."""
+    return st["threads"] * -(-st["blocks"] // st["launch_blocks"]) if st["forms"]["batch"] == "teams" else st["threads"]
 
 
 def make_simulator(a, dp, sp, streams, gpu):
@@ -380,9 +381,9 @@ def run_gb300_queued(a, rank, ws, dp, sp, info, streams, schedule, gpu):
             "vs_baseline": None, "dtype": "u8 nibbles (8 streams per u32)", "data": "synthetic (seeded generator)",
             "config": {"workload": f"{a.workload}: {st['lut_ops']} LUT ops, {streams} streams of log-uniform length "
                                    f"(mean {cyc.mean():.0f}), {s.options()['n_streams']} slots, longest first",
-                       "stream_cycles": int(cyc.sum()), "schedule": a.schedule, "exec_levels": exec_levels(st),
+                       "stream_cycles": int(cyc.sum()), "schedule": a.schedule, "exec_levels": st["forms"]["queue"],
                        "mode": ["persistent", "graph"][s.options()["mode"]],
-                       "blocks": st["blocks"],
+                       "blocks": st["region_items"] if st["forms"]["queue"] == "own streams" else st["blocks"],
                        "threads_per_block": st["threads"],
                        "groups_per_item": st["groups_per_item"], **notes},
             "lut_evals_per_s": total / dev_s * st["lut_ops"],
@@ -599,14 +600,15 @@ def run_gb300(a, rank, ws):
                        "streams": streams, "cycles_per_step": cps, "lut_ops": st["lut_ops"],
                        "partitions": st["partitions"], "groups_per_item": st["groups_per_item"],
                        "mode": ["persistent", "graph"][s.options()["mode"]], "value_pool": a.value_pool,
-                       "smem_per_block": st.get("smem_per_block"), "exec_levels": exec_levels(st), **notes,
-                       "threads_per_block": st["threads"], "blocks": st["blocks"],
+                       "smem_per_block": st.get("smem_per_block"), "exec_levels": st["forms"]["batch"], **notes,
+                       "threads_per_block": threads_per_block(st), "blocks": st["launch_blocks"],
                        "l2": "working set (memories) larger than L2"},
             "lut_evals_per_s": value * st["lut_ops"],
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_source": peak_kind,
-                         "kernel": f"{'regionKernel' if graph else 'cycleKernel'}<{st['streams_per_word']},"
-                                   f"{st['groups_per_item']}>",
+                         "kernel": "ownStreamsKernel<%d>" % st["groups_per_item"] if st["forms"]["batch"] == "own streams"
+                                   else f"{'regionKernel' if graph else 'cycleKernel'}<{st['streams_per_word']},"
+                                        f"{st['groups_per_item']}> ({st['forms']['batch']})",
                          "algorithmic_bytes_per_launch": bytes_launch, "launch_us": launch_s * 1e6,
                          "note": "bound on chip by instruction issue and shared-memory table lookups (profiles/): HBM "
                                  "is not the limit",

@@ -120,7 +120,7 @@ typedef struct tgs_tune_opts {
 
 typedef struct tgs_tune_trial {
   uint32_t groups_per_item, warps_per_block, blocks_per_sm, mode;
-  uint32_t staged;      /* exec levels: 1 staged per level, 2 resident for the launch, 0 read from global memory, 3 warp programs */
+  uint32_t staged;      /* TGS_FORM_* of the trial's launches */
   uint32_t blocks;      /* grid size of the trial */
   float ms_per_cycle;   /* negative: the configuration does not fit */
   uint32_t mpart_lanes, levels_per_barrier;
@@ -320,6 +320,16 @@ int tgs_host_free(void *p);
 int tgs_device_reset(int device);
 
 /* ---- design statistics and launch shape (new) ------------------------- */
+/* where the blocks of a launch read the exec levels */
+enum {
+  TGS_FORM_GLOBAL = 0,            /* level by level from global memory */
+  TGS_FORM_STAGED = 1,            /* staged per level into shared memory */
+  TGS_FORM_RESIDENT = 2,          /* kept in shared memory for the launch */
+  TGS_FORM_PROGRAMS = 3,          /* warp programs read from global memory */
+  TGS_FORM_PROGRAMS_RESIDENT = 4, /* warp programs kept in shared memory for the launch */
+  TGS_FORM_TEAMS = 5,             /* warp programs, an SM's blocks as teams of one block */
+  TGS_FORM_OWN_STREAMS = 6        /* resident warp programs, blocks that own their streams */
+};
 typedef struct tgs_design_stats {
   uint64_t lut_ops;          /* table lookups (lutIndex != 0) */
   uint64_t nop_ops;          /* moves (lutIndex == 0) */
@@ -329,16 +339,21 @@ typedef struct tgs_design_stats {
   uint64_t mem_read_ops, mem_write_ops, vec_ops, vec_read_ops, print_ops, stop_ops;
   uint64_t op_slots;         /* every op slot, 32-bit words of instruction per cycle */
   uint32_t partitions, mparts, max_value_pool, max_exec_levels;
-  uint32_t blocks, threads, groups_per_item, streams_per_word;
+  uint32_t blocks, threads;  /* blocks of work, and threads of each: a launched block runs one, or blocks /
+                                launch_blocks of them side by side (teams) */
+  uint32_t groups_per_item, streams_per_word;
   uint64_t block_barriers, exec_levels;   /* block barriers kept / exec levels, all partitions */
   double makespan[2];        /* scheduled cost of the slowest block per region */
-  uint32_t smem_per_block;   /* dynamic shared memory of a block: table, stage buffers, value pool */
+  uint32_t smem_per_block;   /* dynamic shared memory of a launched block (batch runs): tables, what stays resident,
+                                stage buffers, value pools */
   uint32_t stage_words;      /* words of one exec-level stage buffer (0: levels resident or read from global memory) */
   uint32_t resident_words;   /* words of a block's resident exec levels (0: staged or read from global memory) */
   uint32_t fused_levels;     /* exec levels merged into the block before them (levels_per_barrier > 1) */
   uint32_t program_words;    /* words of the warp programs (0: exec levels resident, staged or global) */
   uint32_t region_items;     /* (partition, group block) items of the larger region */
-  uint32_t reserved[2];
+  uint32_t launch_blocks;    /* grid of a batch run's launch */
+  uint32_t launch_forms;     /* TGS_FORM_* of batch runs (bits 0..7), of queued runs on as many slots (8..15) and of
+                                free running (16..23) with the current options */
 } tgs_design_stats;
 int tgs_get_design_stats(const tgs_sim *h, tgs_design_stats *out);
 

@@ -44,6 +44,7 @@ def test_smaller_second_handle(tmp_path, built, form):
     try:
         for s, dp, sp, stim, ref in runs:
             s.init(0, dp, sp, False, False)
+            assert s.design_stats()["forms"]["batch"] == form
             check(s, stim, ref, 6)
         for s, dp, sp, stim, ref in runs:  # the larger one again, after the smaller one; other cycles: captured anew
             check(s, stim, ref, 6)

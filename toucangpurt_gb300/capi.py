@@ -89,6 +89,10 @@ class GenInfo(C.Structure):
     ]
 
 
+# TGS_FORM_*: where the blocks of a launch read the exec levels
+FORMS = ("global", "staged", "resident", "programs", "resident programs", "teams", "own streams")
+
+
 class DesignStats(C.Structure):
     _fields_ = [
         ("lut_ops", C.c_uint64), ("nop_ops", C.c_uint64), ("writeback_ops", C.c_uint64),
@@ -100,7 +104,7 @@ class DesignStats(C.Structure):
         ("groups_per_item", C.c_uint32), ("streams_per_word", C.c_uint32), ("block_barriers", C.c_uint64),
         ("exec_levels", C.c_uint64), ("makespan", C.c_double * 2), ("smem_per_block", C.c_uint32),
         ("stage_words", C.c_uint32), ("resident_words", C.c_uint32), ("fused_levels", C.c_uint32),
-        ("program_words", C.c_uint32), ("region_items", C.c_uint32), ("reserved", C.c_uint32 * 2),
+        ("program_words", C.c_uint32), ("region_items", C.c_uint32), ("launch_blocks", C.c_uint32), ("launch_forms", C.c_uint32),
     ]
 
 

@@ -288,9 +288,35 @@ uint32_t autoWarps(const DeviceImage &img, uint32_t G, uint32_t spw) {
   return std::clamp<uint32_t>(best, 6, 16);
 }
 
-// tgs_tune_trial.staged: 0 global, 1 staged, 2 resident, 3 warp programs
-uint32_t levelSource(const tgs_sim *h) {
-  return h->lc.lv == kLevelsProgram ? 3u : h->resWords ? 2u : h->stageWords ? 1u : 0u;
+// The form (TGS_FORM_*) in which a run with these flags is launched.  Teams
+// where they are set up; queued streams (whose retirements every block looks
+// for) and micro-partition profiles take the block form.
+uint32_t runForm(const tgs_sim *h, uint32_t flags) {
+  const bool persistent = h->opt.mode != TGS_MODE_GRAPH, profile = (flags & kFlagProfileMP) != 0;
+  if (persistent && h->ownWords && h->ownCounts && !(flags & ~(kFlagStimulus | kFlagDigest | kFlagSlots | kFlagStopExit)))
+    return TGS_FORM_OWN_STREAMS;
+  if (persistent && h->progResWords && !profile) return TGS_FORM_PROGRAMS_RESIDENT;
+  if (h->teams && !(flags & kFlagSlots) && !profile) return TGS_FORM_TEAMS;
+  if (h->lc.lv == kLevelsProgram) return TGS_FORM_PROGRAMS;
+  return h->resWords ? TGS_FORM_RESIDENT : h->stageWords ? TGS_FORM_STAGED : TGS_FORM_GLOBAL;
+}
+
+// The launch of a form.
+LaunchCfg launchCfg(const tgs_sim *h, uint32_t form) {
+  LaunchCfg c = h->lc;
+  if (form == TGS_FORM_OWN_STREAMS) {
+    c.blocks = h->gpad / uint32_t(h->lc.G);
+    c.smem = h->ownSmem;
+  } else if (form == TGS_FORM_PROGRAMS_RESIDENT) {
+    c.lv = kLevelsProgramResident;
+    c.smem = h->progResSmem;
+  } else if (form == TGS_FORM_TEAMS) {
+    c.lv = kLevelsProgramTeams;
+    c.blocks = uint32_t(h->props.multiProcessorCount);
+    c.teams = h->teams;
+    c.smem = h->teamSmem;
+  }
+  return c;
 }
 
 // Whether records of 8 and more levels hold over a quarter of the ops.
@@ -790,26 +816,12 @@ void requireLoaded(tgs_sim *h, bool ordered = false) {
   }
 }
 
-// The launch of a run with these flags: teams where they are set up; queued
-// streams (whose retirements every block looks for) and micro-partition
-// profiles take the block form.
-LaunchCfg launchCfg(const tgs_sim *h, uint32_t flags) {
-  LaunchCfg c = h->lc;
-  if (h->teams && !(flags & (kFlagSlots | kFlagProfileMP))) {
-    c.lv = kLevelsProgramTeams;
-    c.blocks = uint32_t(h->props.multiProcessorCount);
-    c.teams = h->teams;
-    c.smem = h->teamSmem;
-  }
-  return c;
-}
-
 // Graph form: chunks of up to 32 cycles (two region launches and an admit
 // launch per cycle) captured once and replayed.  The kernels read the cycle,
 // the event cursor and the end cycle from device words, so a chunk captured
 // for one call serves every later call with the same launch parameters.
 cudaGraphExec_t graphChunk(tgs_sim *h, const KParams &p, uint32_t k, bool admit) {
-  const LaunchCfg c = launchCfg(h, p.flags);
+  const LaunchCfg c = launchCfg(h, runForm(h, p.flags));
   std::vector<uint8_t> key(sizeof(KParams) + 9 * sizeof(uint32_t));
   std::memcpy(key.data(), &p, sizeof(KParams));
   const uint32_t tail[9] = {k,         admit ? 1u : 0u,    uint32_t(c.spw), uint32_t(c.G), c.blocks,
@@ -876,11 +888,11 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     runGraph(h, c0, n, flags, stopped0);
     return;
   }
-  if (h->ownWords && h->ownCounts && !(flags & ~(kFlagStimulus | kFlagDigest | kFlagSlots | kFlagStopExit))) {
-    LaunchCfg c = h->lc;
-    KParams p = h->kp;
-    c.blocks = p.nBlocks = h->gpad / uint32_t(h->lc.G);
-    c.smem = h->ownSmem;
+  const uint32_t form = runForm(h, flags);
+  const LaunchCfg c = launchCfg(h, form);
+  KParams p = h->kp;
+  if (form == TGS_FORM_OWN_STREAMS) {
+    p.nBlocks = c.blocks;
     p.items = h->ownItems.p;
     p.itemBegin = h->ownBegin.p;
     p.itemRes = h->ownRes.p;
@@ -889,20 +901,13 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     p.resWords = h->ownWords;
     p.resSrc = h->partImages.p;
     TGS_CUDA(launchOwnStreams(c, p, c0, n));
-    h->lastLaunches = 1;
-    return;
-  }
-  if (h->lc.blocks > 1) TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
-  if (h->progResWords && !(flags & kFlagProfileMP)) {
-    LaunchCfg c = h->lc;
-    KParams p = h->kp;
-    c.lv = kLevelsProgramResident;
-    c.smem = h->progResSmem;
-    p.resWords = h->progResWords;
-    p.resSrc = h->partImages.p;
-    TGS_CUDA(launchCycles(c, p, c0, n));
   } else {
-    TGS_CUDA(launchCycles(launchCfg(h, flags), h->kp, c0, n));
+    if (h->lc.blocks > 1) TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
+    if (form == TGS_FORM_PROGRAMS_RESIDENT) {
+      p.resWords = h->progResWords;
+      p.resSrc = h->partImages.p;
+    }
+    TGS_CUDA(launchCycles(c, p, c0, n));
   }
   h->lastLaunches = 1;
 }
@@ -1243,14 +1248,14 @@ int tgs_autotune(tgs_sim *h, const tgs_tune_opts *opts, tgs_tune_trial *trials, 
             if (fits && h->lc.G != int(G)) fits = false;  // fewer groups than G: same as a smaller G
             if (fits && h->lc.blocks == lastBlocks) continue;  // same grid as the previous trial
             if (fits) lastBlocks = h->lc.blocks;
-            tr.blocks = fits ? h->lc.blocks : 0;
-            tr.staged = !fits ? 0u : levelSource(h);
             for (uint32_t mode = 0; mode < 2; ++mode) {
               if (!(modes & (1u << mode))) continue;
               tr.mode = mode;
               tr.ms_per_cycle = -1.f;
               if (fits) {
                 h->opt.mode = mode;
+                tr.staged = runForm(h, 0);
+                tr.blocks = launchCfg(h, tr.staged).blocks;
                 resetState(h);
                 fillParams(h);
                 runTimed(h, 0, warm, 0);
@@ -1296,8 +1301,8 @@ int tgs_autotune(tgs_sim *h, const tgs_tune_opts *opts, tgs_tune_trial *trials, 
             fits = false;
           }
           if (fits) {
-            tr.blocks = h->lc.blocks;
-            tr.staged = levelSource(h);
+            tr.staged = runForm(h, 0);
+            tr.blocks = launchCfg(h, tr.staged).blocks;
             resetState(h);
             fillParams(h);
             runTimed(h, 0, warm, 0);
@@ -2156,7 +2161,12 @@ extern "C" int tgs_get_design_stats(const tgs_sim *h, tgs_design_stats *o) {
     o->region_items = h->regionItems;
     o->makespan[0] = h->sched.makespan[0];
     o->makespan[1] = h->sched.makespan[1];
-    o->smem_per_block = uint32_t(h->lc.smem);
+    const uint32_t batch = runForm(h, kFlagStimulus | kFlagDigest);
+    const LaunchCfg c = launchCfg(h, batch);
+    o->smem_per_block = uint32_t(c.smem);
+    o->launch_blocks = c.blocks;
+    o->launch_forms = batch | runForm(h, kFlagStimulus | kFlagDigest | kFlagSlots) << 8 |
+                      runForm(h, kFlagCountCycles | kFlagProfile) << 16;
     o->stage_words = h->stageWords;
     o->resident_words = h->resWords;
   });

@@ -163,6 +163,8 @@ class Simulator:
         check(lib().tgs_get_design_stats(self._h, C.byref(st)))
         d = {f: getattr(st, f) for f, _ in capi.DesignStats._fields_ if f not in ("reserved", "makespan")}
         d["makespan"] = [st.makespan[0], st.makespan[1]]
+        # the launch form by kind of run
+        d["forms"] = {k: capi.FORMS[st.launch_forms >> 8 * i & 255] for i, k in enumerate(("batch", "queue", "free"))}
         return d
 
     # -- state --------------------------------------------------------------
