@@ -58,6 +58,9 @@ def _same(got, lens, ref):
     ("four", 9, dict(resident_netlist=2), "global", "global", "global"),
     ("four", 9, dict(resident_netlist=3), "staged", "staged", "staged"),
     ("two", 2500, dict(groups_per_item=4, warps_per_block=5), "teams", "programs", "teams"),
+    # the graph form: teams where a region has more items than blocks
+    ("two", 2500, dict(groups_per_item=4, warps_per_block=5, mode=1), "programs", "programs", "programs"),
+    ("two", 2500, dict(groups_per_item=2, warps_per_block=5, blocks_per_sm=2, mode=1), "teams", "programs", "teams"),
 ])
 def test_stats_name_the_launch(designs, name, streams, options, batch, queue, free):
     dp, sp = designs[name][:2]

@@ -290,13 +290,20 @@ uint32_t autoWarps(const DeviceImage &img, uint32_t G, uint32_t spw) {
 
 // The form (TGS_FORM_*) in which a run with these flags is launched.  Teams
 // where they are set up; queued streams (whose retirements every block looks
-// for) and micro-partition profiles take the block form.
+// for) and micro-partition profiles take the block form.  So does the graph
+// form unless a region has more items than blocks: each of its launches, two a
+// cycle, writes the nibble table anew (4 us), which only launches of several
+// items per block win back.  Blocks / teams, ms: 30 cycles of a 300K-LUT design
+// x 128 streams (296 items) 1.37 / 1.59, 100 cycles of the 4K-LUT design x 4,000
+// (250) 2.56 / 3.18, 8 cycles of a mixed 1M-LUT design x 256 (512) 2.63 / 2.78;
+// 20 cycles of a 1M-LUT design x 320 streams (1,280 items, 760 blocks) 3.13 /
+// 3.02, 10 cycles of a 4M-LUT design x 256 (2,048) 4.93 / 4.45.
 uint32_t runForm(const tgs_sim *h, uint32_t flags) {
   const bool persistent = h->opt.mode != TGS_MODE_GRAPH, profile = (flags & kFlagProfileMP) != 0;
   if (persistent && h->ownWords && h->ownCounts && !(flags & ~(kFlagStimulus | kFlagDigest | kFlagSlots | kFlagStopExit)))
     return TGS_FORM_OWN_STREAMS;
   if (persistent && h->progResWords && !profile) return TGS_FORM_PROGRAMS_RESIDENT;
-  if (h->teams && !(flags & kFlagSlots) && !profile) return TGS_FORM_TEAMS;
+  if (h->teams && !(flags & kFlagSlots) && !profile && (persistent || h->regionItems > h->lc.blocks)) return TGS_FORM_TEAMS;
   if (h->lc.lv == kLevelsProgram) return TGS_FORM_PROGRAMS;
   return h->resWords ? TGS_FORM_RESIDENT : h->stageWords ? TGS_FORM_STAGED : TGS_FORM_GLOBAL;
 }
