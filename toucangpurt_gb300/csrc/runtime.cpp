@@ -386,6 +386,12 @@ void configure(tgs_sim *h) {
         G >>= 1;
     }
     while (G > 1 && uint32_t(G) > h->groups) G >>= 1;
+    // by default no more groups than a block's shared memory has value pools for
+    const int lv = program ? kLevelsProgram : kLevelsStaged;
+    while (!o.groups_per_item && G > 1 &&
+           kLutTablePadded + size_t(h->img.maxVpSlots) * size_t(G) * 4 >
+               std::min(mostSharedMemory(h, cycleKernelFor(8, G, lv)), mostSharedMemory(h, regionKernelFor(8, G, lv))))
+      G >>= 1;
   }
   h->gpad = (h->groups + G - 1) / G * G;
   SchedOpts so;
