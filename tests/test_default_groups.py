@@ -33,3 +33,36 @@ def test_large_value_pools(tmp_path, built, value_pool):
             s.set_options(groups_per_item=4)
     ref = pyoracle.OracleDesign(dp, sp).run(np.full(24, 3, np.uint32), stim)
     np.testing.assert_array_equal(got.final_reg_digest[:24], ref["final_reg_digest"])
+
+
+@pytest.fixture(scope="module")
+def cones(tmp_path_factory, built):
+    """Records of several levels, 18 partitions in a region."""
+    d = tmp_path_factory.mktemp("cones")
+    dp, sp = d / "d.bin", d / "d.sym"
+    info = sim.generate(dp, sp, **workloads.design_config("scale", seed=15, n_lut=14_000, luts_per_part=400, levels=9,
+                                                          ff_bits=2_000, n_vec_ops=8, n_mems=2, mem_depth=64,
+                                                          cone_depth=3))
+    return dp, sp, info
+
+
+# both sides of two items of one group per SM and of three items of two groups
+@pytest.mark.parametrize("mode", [0, 1])
+def test_records_of_several_levels(cones, mode):
+    dp, sp, info = cones
+    stim = sim.StimulusSpec(3, info["pi_ids"], info["pi_bits"])
+    ref = pyoracle.OracleDesign(dp, sp).run(np.full(40, 5, np.uint32), stim)["final_reg_digest"]
+    seen = set()
+    with sim.Simulator(mode=mode) as s:
+        s.init(0, dp, sp, False, False)
+        parts = s.design_stats()["region_items"]  # one stream: an item per partition
+        for n in (40, 128, 136, 256, 400, 408, 520):
+            groups = -(-n // 8)
+            want = 4 if parts * -(-groups // 2) > 3 * 152 else 2 if parts * groups > 2 * 152 else 1
+            if want == 2 and 6 * (groups + groups % 2) > 7 * groups:  # more padding than a sixth
+                want = 1
+            got = s.batch_run(np.full(n, 5, np.uint32), stim)
+            assert s.design_stats()["groups_per_item"] == want, n
+            seen.add(want)
+            np.testing.assert_array_equal(got.final_reg_digest[:40], ref[:min(n, 40)])
+    assert seen == {1, 2, 4}

@@ -326,14 +326,14 @@ LaunchCfg launchCfg(const tgs_sim *h, uint32_t form) {
   return c;
 }
 
-// Whether records of 8 and more levels hold over a quarter of the ops.
-bool chainHeavy(const DeviceImage &img) {
+// Whether records of at least `depth` levels hold over a quarter of the ops.
+bool deepRecords(const DeviceImage &img, uint32_t depth) {
   uint64_t ops = 0, deep = 0;
   for (const auto &part : img.mp)
     for (const auto &lv : part)
       for (const auto &m : lv) {
         ops += m.feat.ops;
-        if (m.feat.depth >= 8) deep += m.feat.ops;
+        if (m.feat.depth >= depth) deep += m.feat.ops;
       }
   return 4 * deep > ops;
 }
@@ -367,23 +367,36 @@ void configure(tgs_sim *h) {
     } else {
       // default: 4 groups per item (a record's decoding is paid once for all
       // of them) while a region has an item per SM and padding adds at most a
-      // sixth to the groups; fewer for few, narrow partitions.  Two items per
-      // SM where long middle-level chains hold a quarter of the ops (one warp
-      // runs a chain while the block waits) and for levels that are not read
-      // as warp programs.  30 cycles, ms with 1 / 2 / 4 groups per item:
-      // 1M-LUT design x 64 streams 1.66 / 1.54 / 1.36 (256 items with 4);
-      // 300K-LUT x 256 1.84 / 1.56 / 1.33 (296), x 128 1.06 / 0.91 / 1.03
-      // (148: 2 groups); 1M-LUT x 40, 5 groups, 1.26 / 1.31 / 1.36; mixed
-      // 1M-LUT design with chains x 64 5.97 / 6.71 / 7.76 (512, 256, 128).
+      // sixth to the groups; fewer for few, narrow partitions.  30 cycles, ms
+      // with 1 / 2 / 4 groups per item: 1M-LUT design x 64 streams 1.66 / 1.54
+      // / 1.36 (256 items with 4); 300K-LUT x 256 1.84 / 1.56 / 1.33 (296), x
+      // 128 1.06 / 0.91 / 1.03 (148: 2 groups); 1M-LUT x 40, 5 groups, 1.26 /
+      // 1.31 / 1.36.
+      // Two items per SM where long middle-level chains hold a quarter of the
+      // ops (one warp runs a chain while the block waits) and for levels that
+      // are not read as warp programs: mixed 1M-LUT design with chains x 64
+      // 5.97 / 6.71 / 7.76 (512, 256, 128).
+      // Where records of several levels do (cones), which one warp takes level
+      // after level for all its groups: twice the groups only from more than
+      // two items per SM of one group, or three of two, on.  40 cycles, ms
+      // persistent with 1 / 2 / 4: 100K-LUT design, cones of 3, x 136 (289
+      // items of one group) 0.95 / 1.14 / 1.31, x 168 (357) 1.40 / 1.15 / 1.33,
+      // x 400 (425 of two) 2.23 / 1.67 / 1.72, x 520 (561) 2.53 / 1.82 / 1.72;
+      // graph form 1.37 / 1.50 / 1.69, 1.46 / 1.52 / 1.70, 2.78 / 1.80 / 2.02,
+      // 3.05 / 2.07 / 2.07.  20 cycles, 250K-LUT design, cones of 4: x 72 (288
+      // of one) 0.61 / 0.70 / 0.66, x 136 (544) 0.97 / 0.73 / 0.96, x 200 (416
+      // of two) 1.14 / 0.85 / 0.99, x 256 (512) 1.47 / 1.15 / 1.01.
       size_t parts = 1;
       for (auto &r : h->design.regionPartitionIds) parts = std::max(parts, r.size());
       const size_t sms = size_t(std::max(1, h->props.multiProcessorCount));
-      const size_t want = program && !chainHeavy(h->img) ? sms : 2 * sms;
+      const bool chains = !program || deepRecords(h->img, 8), cones = !chains && deepRecords(h->img, 2);
       const bool pad = program;  // staged levels: any padding, as they were measured
+      auto items = [&](int g) { return parts * ((h->groups + g - 1) / g); };
+      auto enough = [&](int g) {
+        return cones ? items(g / 2) > (g == 2 ? 2 : 3) * sms : items(g) >= (chains ? 2 : 1) * sms;
+      };
       G = 4;
-      while (G > 1 && (parts * ((h->groups + G - 1) / G) < want ||
-                       (pad && 6 * ((h->groups + G - 1) / G * G) > 7 * h->groups)))
-        G >>= 1;
+      while (G > 1 && (!enough(G) || (pad && 6 * ((h->groups + G - 1) / G * G) > 7 * h->groups))) G >>= 1;
     }
     while (G > 1 && uint32_t(G) > h->groups) G >>= 1;
     // by default no more groups than a block's shared memory has value pools for
