@@ -1791,20 +1791,23 @@ __device__ __forceinline__ bool gridSync(const KParams &p, uint32_t &gen) {
     const uint32_t target = (gen + 1u) * gridDim.x;
     // the release orders the block's writes (the block barrier above put them
     // before this thread's) before the arrival, the acquiring load the block's
-    // later reads after it; the error word and the time are looked at every 64
-    // polls (two full fences, the error word and the timer on every poll took
-    // 1,024 queued streams of the 4K-LUT design 39.3 ms, this 37.0)
+    // later reads after it.  The error word is read beside the first of every
+    // 64 polls, so that a launch ends at the first barrier that waits after an
+    // error; the time is looked at after the last of them (two full fences,
+    // the error word and the timer on every poll took 1,024 queued streams of
+    // the 4K-LUT design 39.3 ms, this 37.0)
     uint32_t seen;
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(seen) : "l"(p.barrier) : "memory");
     ++seen;
     unsigned long long t0 = 0;
     for (uint32_t spin = 1; int32_t(seen - target) < 0; ++spin) {
+      const uint32_t bad = (spin & 63u) == 1u ? *static_cast<volatile uint32_t *>(p.err) : 0u;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(p.barrier) : "memory");
-      if ((spin & 63u) != 0u || int32_t(seen - target) >= 0) continue;
-      if (*static_cast<volatile uint32_t *>(p.err) != 0u) {
+      if (bad != 0u) {
         ok = 0;
         break;
       }
+      if ((spin & 63u) != 0u || int32_t(seen - target) >= 0) continue;
       if (t0 == 0) {
         t0 = gtimer();
       } else if (gtimer() - t0 > p.timeoutNs) {
