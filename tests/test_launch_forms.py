@@ -157,3 +157,26 @@ def test_resident_programs_with_stops(designs, n, stop_exit):
         s.init(0, dp, sp, False, False)
         assert s.design_stats()["forms"]["batch"] == "resident programs"
         _same(s.batch_run(cyc, stim, stop_exit=stop_exit, cycle_digests=True), lens, ref)
+
+
+# eval() takes its outcome from page-locked words, in which every block that
+# owns its streams puts what it has seen; the graph form copies the stop flags
+@pytest.mark.parametrize("groups,n", [(1, 17), (2, 40)])
+def test_own_streams_eval_outcome(designs, groups, n):
+    dp, sp, info, _ = designs["one"]
+    stim = sim.StimulusSpec(5, info["pi_ids"], info["pi_bits"])
+    table = sim.stimulus_table(stim, n, 0, 30)
+    for only in (0, n // 2, n - 1):  # the stream that gets inputs, in the first, a middle and the last block
+        out = []
+        for mode in (capi.MODE_PERSISTENT, capi.MODE_GRAPH):
+            with sim.Simulator(n_streams=n, groups_per_item=groups, mode=mode) as s:
+                s.init(0, dp, sp, False, False)
+                assert s.design_stats()["forms"]["batch"] == ("programs" if mode else "own streams")
+                stops = []
+                for c in range(30):
+                    pool = s.reg_pool(only)
+                    pool[info["pi_ids"]] = table[c, :, only]
+                    s.write_reg_pool(pool, only)
+                    stops.append(s.eval())
+                out.append((stops, s.digest(only), s.eval_done()))
+        assert out[0] == out[1]

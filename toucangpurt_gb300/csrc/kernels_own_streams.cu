@@ -158,7 +158,10 @@ __global__ void __launch_bounds__(kResidentThreads) ownStreamsKernel(const KPara
   __shared__ uint32_t itemLists[2 * kItemListWords];
   __shared__ OwnStreams<G> o;
   BlockSmem b;
-  if (!setupBlock<G, kLevelsProgramResident>(p, smem, stageMbar, b, -1)) return;
+  if (!setupBlock<G, kLevelsProgramResident>(p, smem, stageMbar, b, -1)) {
+    if (threadIdx.x == 0) p.status[0] = kErrTimeout;
+    return;
+  }
   loadItemLists(p, b, itemLists);
   const bool slots = (p.flags & kFlagSlots) != 0, stopExit = (p.flags & kFlagStopExit) != 0;
   const bool digest = (p.flags & kFlagDigest) != 0, stim = (p.flags & kFlagStimulus) != 0;
@@ -231,6 +234,17 @@ __global__ void __launch_bounds__(kResidentThreads) ownStreamsKernel(const KPara
   if (!slots)
     for (uint32_t s = tid; s < N; s += blockDim.x)
       if (s0 + s < p.nStreams) p.roll[s0 + s] = o.roll[s];
+  // the run's outcome for the host (zeroed before the launch): each block adds
+  // what it has seen, the block that raised an error that one at least
+  uint32_t any = 0;
+  for (uint32_t s = tid; s < N; s += blockDim.x)
+    if (s0 + s < p.nStreams) any |= __ldcg(p.stop + s0 + s);
+  const int stopped = __syncthreads_or(int(any));
+  if (tid == 0) {
+    const uint32_t err = __ldcg(p.err);
+    if (stopped) p.status[1] = 1u;
+    if (err != 0u) p.status[0] = err;
+  }
 }
 
 template <int G>

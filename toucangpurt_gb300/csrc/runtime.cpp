@@ -926,6 +926,8 @@ void runCycles(tgs_sim *h, uint32_t c0, uint32_t n, uint32_t flags) {
     p.resCopyBegin = h->ownCopyBegin.p;
     p.resWords = h->ownWords;
     p.resSrc = h->partImages.p;
+    h->status[0] = kErrNone;  // its blocks only write what is not so
+    h->status[1] = 0;
     TGS_CUDA(launchOwnStreams(c, p, c0, n));
   } else {
     if (h->lc.blocks > 1) TGS_CUDA(cudaMemsetAsync(h->barrier.p, 0, 2 * sizeof(uint32_t), h->stream));
