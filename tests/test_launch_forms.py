@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from oracle import pyoracle
+from tests import designlib as dl
 from toucangpurt_gb300 import capi, sim, workloads
 
 pytestmark = pytest.mark.gpu
@@ -180,3 +181,24 @@ def test_own_streams_eval_outcome(designs, groups, n):
                     stops.append(s.eval())
                 out.append((stops, s.digest(only), s.eval_done()))
         assert out[0] == out[1]
+
+
+# memories that hold bytes of 0x80 and above, whose digest terms carry out of
+# the low byte; sizes off the 16 bytes that the retirements read at a time
+@pytest.mark.parametrize("size", [40, 64, 77])
+@pytest.mark.parametrize("mode,form", [(0, "own streams"), (1, "programs")])
+def test_retired_memories_of_any_bytes(tmp_path, built, size, mode, form):
+    zero = [dl.MPart(top=[], wbs=[dl.wb(0, 64 + i) for i in range(32)])]
+    p0 = dl.Part(vp_size=160, reg_reads=[(i, 16 + i) for i in range(16)], levels=[zero], exg_write=(0, 64, 32))
+    p1 = dl.Part(vp_size=64, exg_reads=[(i, 16 + i) for i in range(32)], levels=[], reg_write=(16, 16, 32))
+    for fill in (np.arange(size) * 37 % 256, np.arange(size) % 128):
+        d = dl.Design(reg_pool=64, mem_pool=size, exg_pool=32, parts=[p0, p1], regions=[[0], [1]],
+                      mem_init=fill.astype(np.uint8).tobytes())
+        d.write(tmp_path / "d.bin")
+        with np.errstate(over="ignore"):
+            want = sim.mix64(np.arange(size, dtype=np.uint64) << np.uint64(8) | fill.astype(np.uint64)).sum(dtype=np.uint64)
+        with sim.Simulator(groups_per_item=1, mode=mode, validate=0) as s:  # the static checks want nibbles
+            s.init(0, tmp_path / "d.bin", None, False, False)
+            got = s.batch_run((np.arange(50) % 9 + 1).astype(np.uint32), slots=24)
+            assert s.design_stats()["forms"]["queue"] == form
+        np.testing.assert_array_equal(got.final_mem_digest, np.full(50, want, np.uint64))

