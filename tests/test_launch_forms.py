@@ -53,6 +53,10 @@ def _same(got, lens, ref):
     ("one", 1, {}, "resident programs", "resident programs", "resident programs"),
     ("one", 9, {}, "own streams", "own streams", "resident programs"),
     ("one", 9, dict(mode=1), "programs", "programs", "programs"),
+    # 152 and 153 blocks of one group, one per SM asked for
+    ("one", 8 * 152, dict(groups_per_item=1, blocks_per_sm=1), "own streams", "own streams", "resident programs"),
+    ("one", 8 * 153, dict(groups_per_item=1, blocks_per_sm=1), "resident programs", "resident programs", "resident programs"),
+    ("one", 8 * 153, dict(groups_per_item=1), "own streams", "own streams", "resident programs"),
     ("four", 9, {}, "resident programs", "resident programs", "resident programs"),
     ("four", 9, dict(warps_per_block=17), "programs", "programs", "programs"),
     ("four", 9, dict(resident_netlist=1), "resident", "resident", "resident"),
@@ -70,6 +74,7 @@ def test_stats_name_the_launch(designs, name, streams, options, batch, queue, fr
         st = s.design_stats()
     assert st["forms"] == {"batch": batch, "queue": queue, "free": free}
     assert st["launch_blocks"] == (152 if batch == "teams" else st["blocks"])
+    assert not options.get("blocks_per_sm") or st["launch_blocks"] <= 152 * options["blocks_per_sm"]
     # the truth table and a value pool for every block of work in a launched block
     pools = -(-st["blocks"] // st["launch_blocks"])
     assert st["smem_per_block"] >= 4642 + pools * 4 * st["max_value_pool"] * st["groups_per_item"]

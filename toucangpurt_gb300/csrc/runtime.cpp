@@ -598,9 +598,11 @@ void configure(tgs_sim *h) {
       h->resCopyBegin.upload(resBegin, h->stream);
       // One partition per region: blocks that own their streams, one per
       // group block (with more partitions a group block's items are spread
-      // over several blocks instead, which the grid barrier then ties)
+      // over several blocks instead, which the grid barrier then ties).  They
+      // are launched all at once: not beyond the blocks per SM asked for.
       const auto &rp = h->design.regionPartitionIds;
-      if (h->spw == 8 && nGB > 1 && rp.size() == 2 && rp[0].size() == 1 && rp[1].size() == 1) {
+      const bool allowed = !o.blocks_per_sm || nGB <= uint64_t(o.blocks_per_sm) * h->props.multiProcessorCount;
+      if (allowed && h->spw == 8 && nGB > 1 && rp.size() == 2 && rp[0].size() == 1 && rp[1].size() == 1) {
         const uint32_t p0 = rp[0][0], p1 = rp[1][0], w0 = h->sched.imageWords[p0], w1 = h->sched.imageWords[p1];
         void *fnOwn = ownStreamsKernelFor(G);
         const uint32_t ownWords = w0 + w1 + 64u * kProgAhead;
