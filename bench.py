@@ -548,14 +548,16 @@ def run_gb300(a, rank, ws):
     # the dominant kernel: one regionKernel launch per region and cycle (graph
     # form) or one cycleKernel launch per step (persistent form); the device
     # time of a step is those launches (advance and stimulus launches are
-    # ~0.01 % of it, profiles/)
+    # ~0.01 % of it).  The profiled figures are the region kernel's, whose
+    # launches are small enough to capture: a step of the persistent form runs
+    # the same regions, 2 a cycle
     graph = s.options()["mode"] == 1
     launches_step = 2 * cps if graph else 1
     bytes_launch = algorithmic_bytes(st, streams, cps) / launches_step
     launch_s = dev_ms / 1000.0 / a.steps / launches_step
     achieved = bytes_launch / launch_s / 1e9
     prof = a.workload == "largest" and streams == 64
-    traffic = int(profiled("traffic_bytes_per_launch")) if prof and profiled("traffic_bytes_per_launch") else None
+    traffic = int(profiled("traffic_bytes_per_launch")) * 2 * cps // launches_step if prof and profiled("traffic_bytes_per_launch") else None
     cpu = parity = plain = refk = None
     if rank == 0 and ws == 1 and not a.no_cpu_baseline:
         from oracle import pyoracle

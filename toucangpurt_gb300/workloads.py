@@ -89,9 +89,9 @@ def bench_simulator(name: str, design, symbols, *, streams: int | None = None, g
                     profile_cycles: int = 20, epochs: int = 40, seed: int = 5, samples: int = 200_000, **options):
     """A simulator loaded and configured the way the benchmark runs a
     workload: `streams` resident streams (default: the workload's count),
-    the CUDA-graph form unless the exec levels stay resident in shared
-    memory or no block has more than one item of a region (then one
-    persistent launch), and for more than one stream the
+    one persistent launch for warp programs and for exec levels that stay
+    resident in shared memory, the CUDA-graph form for staged or global
+    levels, and for more than one stream the
     learned schedule (every micro-partition profiled for `profile_cycles`
     cycles, repeated until about `samples` (features, clock64 cycles) samples
     are collected, the cost model trained on them).  Further tgs_options
@@ -111,10 +111,12 @@ def bench_simulator(name: str, design, symbols, *, streams: int | None = None, g
     s.init(gpu, design, symbols, False, False)
     notes = {"schedule": schedule}
     st = s.design_stats()
-    if mode == "auto" and (st["resident_words"] or (st["program_words"] and st["region_items"] <= st["blocks"])):
-        # resident levels are loaded once per run; with no more than one item per block a region is one chain of
-        # levels, which a launch per region lengthens (16M-LUT design, one stream: 12.1 ms persistent, 13.1 graph;
-        # 64 streams, three items per block: 48.8 and 47.8)
+    if mode == "auto" and (st["resident_words"] or st["program_words"]):
+        # resident levels are loaded once per run, and so are the tables of warp programs, whose graph form sets a
+        # block up twice a cycle.  Persistent / graph, ms with rolling digests: 50 cycles of the 16M-LUT design x 1
+        # 4.32 / 4.48, x 64 22.52 / 23.13; of the 1M-LUT design x 64 2.41 / 2.64, x 256 5.99 / 6.69; 20 cycles of the
+        # mixed 4M-LUT design x 1 2.19 / 2.23, x 256 15.69 / 15.93.  The graph form is ahead for mixed designs with no
+        # more items of a region than blocks (x 64 6.73 / 6.37) and behind for others of that kind.
         s.set_options(mode=capi.MODE_PERSISTENT)
     if schedule == "learned":
         t0 = time.perf_counter()
