@@ -94,7 +94,7 @@ constexpr uint32_t kDigestSparse = 16;  // lanes of a warp that differ, up to wh
 __global__ void __launch_bounds__(kDigestThreads, 4)
     memDigestKernel(const uint8_t *__restrict__ mems, unsigned long long stride, uint32_t size, uint32_t nStreams,
                     const uint8_t *__restrict__ image, unsigned long long *__restrict__ out) {
-  __shared__ unsigned long long sum[kDigestThreads / 32][kDigestStreams];  // per warp: stream's sum less the first stream's (wrapping)
+  __shared__ unsigned long long sum[kDigestThreads / 32][kDigestStreams];  // per warp: stream's sum less ref's (wrapping)
   __shared__ unsigned long long sum0;
   __shared__ uint32_t piece[kDigestThreads / 32u][kDigestStreams][3], queue[kDigestThreads / 32u][kDigestQueue];
   const uint32_t s0 = blockIdx.y * kDigestStreams, ns = min(kDigestStreams, nStreams - s0);
@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(kDigestThreads, 4)
   }
 }
 
-// The same for pools that are not 16-byte aligned (caller-owned pools).
+// The same a byte a thread: for small pools, and for pools that are not 16-byte
+// aligned (caller-owned pools).
 __global__ void memDigestBytesKernel(const uint8_t *__restrict__ mems, unsigned long long stride, uint32_t size,
                                      uint32_t nStreams, unsigned long long *__restrict__ out) {
   const uint32_t s = blockIdx.y;
@@ -438,7 +439,16 @@ cudaError_t launchRegDigestOne(const uint32_t *regs, uint32_t slots, uint32_t gp
 cudaError_t launchMemDigest(const uint8_t *mems, unsigned long long stride, uint32_t size, uint32_t nStreams,
                             const uint8_t *image, unsigned long long *out, cudaStream_t st) {
   if (size == 0 || nStreams == 0) return cudaSuccess;
-  if (((reinterpret_cast<uintptr_t>(mems) | (nStreams > 1 ? stride : 0ull)) & 15u) != 0u) {
+  // Small pools by bytes: a block that takes 64 pools one after another is
+  // slower than a thread per byte while those leave the GPU room.  us, by 16
+  // bytes / by bytes, 1 % of the bytes different: 1 pool of 8 KiB 4.3 / 3.6, 64
+  // KiB 6.3 / 4.2, 128 KiB 6.2 / 6.3; 64 pools of 8 KiB 37 / 8, 32 KiB 45 / 35,
+  // 64 KiB 45 / 76; 1,000 pools of 4 KiB 41 / 25, 8 KiB 47 / 51 (equal pools 10
+  // by 16 bytes at any of these sizes; wholly different ones 70 up to 32 KiB,
+  // 129 for 64 pools of 64 KiB).
+  const unsigned long long total = (unsigned long long)size * nStreams;
+  const bool small = total <= (128u << 10) || (size <= (32u << 10) && total <= (4u << 20));
+  if (small || ((reinterpret_cast<uintptr_t>(mems) | (nStreams > 1 ? stride : 0ull)) & 15u) != 0u) {
     dim3 grid(std::max<uint32_t>(1, std::min<uint32_t>(1024, (size + 255) / 256)), nStreams);
     memDigestBytesKernel<<<grid, 256, 0, st>>>(mems, stride, size, nStreams, out);
     return cudaGetLastError();
