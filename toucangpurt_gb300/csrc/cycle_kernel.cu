@@ -1,8 +1,8 @@
 // Small kernels of the cycle loop (graph-form admission, stimulus, cycle
 // counter), state utilities, and the host-side launch wrappers.  The cycle
-// and region kernels are instantiated in kernels_{persistent,region}_
-// {staged,resident}.cu, one translation unit each, so the build compiles
-// them in parallel.
+// and region kernels are instantiated in kernels_{persistent,region}_*.cu, one
+// translation unit for each source of exec levels, and kernels_own_streams.cu,
+// so the build compiles them in parallel.
 #include "cycle_kernel.cuh"
 
 namespace tgs {

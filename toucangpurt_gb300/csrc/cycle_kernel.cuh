@@ -1,6 +1,8 @@
 // GB300 (sm_103a) cycle kernel of the Toucan netlist evaluation: the device
-// code shared by the translation units that instantiate its kernels
-// (cycle_kernel.cu and kernels_{persistent,region}_{staged,resident}.cu).
+// code shared by the translation units that instantiate its kernels: one for
+// each source of exec levels of the persistent and the region kernel
+// (kernels_{persistent,region}_*.cu: staged, resident, warp programs streamed,
+// resident or run by teams), kernels_own_streams.cu and cycle_kernel.cu.
 //
 // Restates the reference device code (src/SimEval.cu:304-1056) for many
 // stimulus streams at once:
@@ -1025,10 +1027,12 @@ __device__ __forceinline__ void runLevelsSingle(const KParams &p, const PartDesc
 // instructions of a 32-lane, 4-group record on these (16M-LUT design x 64
 // streams; without any table lookup they still took 42 of 62 ms); a record now
 // takes 225, and a region 135 M instead of 229 M.  Bound now by the
-// shared-memory pipe (bank conflicts of random table reads and operands, 78-83 %
-// of its cycles).  Per 100 cycles: 61.0 -> 47.8 ms; 1M-LUT design x 64 streams
-// 7.8 -> 5.6 ms, one stream 300 cycles 7.9 -> 6.0 ms; 4K-LUT design, one stream,
-// 1,000 cycles (levels resident before) 9.4 -> 6.4 ms.
+// shared-memory pipe in separate blocks (bank conflicts of random table reads
+// and operands, 78-83 % of its cycles), by that pipe, the ALU and issue together
+// in teams (lookupIn).  Per 100 cycles, in separate blocks: 61.0 -> 47.8 ms;
+// 1M-LUT design x 64 streams 7.8 -> 5.6 ms, one stream 300 cycles 7.9 -> 6.0
+// ms; 4K-LUT design, one stream, 1,000 cycles (levels resident before) 9.4 ->
+// 6.4 ms.
 struct ProgOps {
   uint32_t aA, aB, aC, aR, lut;  // operand and result addresses of the item's first group, lut field
 };

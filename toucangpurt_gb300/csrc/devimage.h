@@ -85,8 +85,8 @@ static_assert(sizeof(PartDesc) == 96, "PartDesc size");
 // offset relative to the block and a range of stream groups][micro-partition
 // records, once each, in warp order].  KParams::levelDesc
 // holds (block offset, block words) per level; PartDesc::schedOff indexes
-// the partition's first level there.  A block is staged into shared memory
-// with one bulk async copy while the previous level computes, or, when the
+// the partition's first level there.  A block is staged into shared memory by
+// 16-byte asynchronous copies while the previous level computes, or, when the
 // levels of every partition a block evaluates fit in its shared memory, they
 // are copied there once per launch and stay resident (a partition's level
 // blocks are contiguous in KParams::sched).

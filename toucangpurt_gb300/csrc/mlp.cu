@@ -91,9 +91,10 @@ __global__ void __launch_bounds__(128) mlpForwardKernel(const float *__restrict_
 // weight gradients are dot products over the tile's samples, summed per tile
 // and then over the block's tiles in registers, and added to global memory
 // once per block.  Bound by FP32 FMA issue and the shared loads beside it.
-// tgs_mlp_grad, host arrays in and out: 200,000 samples 2,701 -> 582 us (about
-// 430 us of it copies and allocations), 600,000 7,504 -> 1,072 us, 1,024
-// (a training batch) 230 -> 216 us; error against 64 bits unchanged (7e-7).
+// tgs_mlp_grad, host arrays in and out: 200,000 samples 2,699 -> 530 us (about
+// 430 us of it copies and allocations), 600,000 7,539 -> 1,109 us, 1,024 226 ->
+// 218 us; the kernel alone 20,000 samples 244 -> 36 us, 1,024 (a training
+// batch) 24 -> 16.5; error against 64 bits unchanged (7e-7).
 constexpr uint32_t kTile = 64;     // samples
 constexpr int kRow = 68;           // floats of a shared row of 64 (16-byte aligned, rows 4 banks apart)
 constexpr int tW1 = 0, tW2t = tW1 + kIn * kRow, tW2 = tW2t + kH * kRow, tB1 = tW2 + kH * kRow, tB2 = tB1 + kH,
