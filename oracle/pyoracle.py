@@ -1,7 +1,7 @@
 """ctypes binding of the CPU oracle (oracle/toucan_oracle.h).
 
 TEST INFRASTRUCTURE ONLY: used by tests/, the smoke check and bench.py's
-CPU-baseline leg as the checker; the product never imports it.
+CPU-baseline leg; the product never imports it.
 """
 from __future__ import annotations
 

@@ -1,7 +1,7 @@
 // CPU oracle for the Toucan per-cycle netlist evaluation.
 //
-// TEST INFRASTRUCTURE ONLY (see toucan_oracle.h): the checker for the GPU
-// path and the timed CPU baseline, never part of the product.
+// TEST INFRASTRUCTURE ONLY (see toucan_oracle.h): what the GPU path is compared with
+// and the timed CPU baseline, never part of the product.
 //
 // Parity status: the design-file parser and Init/Randomize are pinned against
 // the reference's own Serializer.cpp / SimInit.cpp compiled from source

@@ -1,6 +1,6 @@
 /* CPU oracle for the Toucan per-cycle netlist evaluation.
  *
- * TEST INFRASTRUCTURE ONLY.  This library is the checker: tests/, the smoke
+ * TEST INFRASTRUCTURE ONLY.  The GPU path is compared with it: tests/, the smoke
  * entry point and the CPU-baseline leg of bench.py may load it; the product
  * (toucangpurt_gb300) never links, loads or calls it.
  *
